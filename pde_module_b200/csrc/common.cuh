@@ -167,6 +167,16 @@ __device__ __forceinline__ float step_time(double t0, double tstep, int n) {
   return __double2float_rn(__dadd_rn(t0, __dmul_rn((double)n, tstep)));
 }
 
+// Boundary value of one group at time t (boundary_functions.py:32-45, 77-92).
+__device__ __forceinline__ float bc_value(int func, float value, float t_max, const float* t_dev) {
+  if (func == PDE_BC_FUNC_RAMP) {
+    float t = t_dev ? *t_dev : 0.0f;
+    float ramp = fminf(__fdiv_rn(t, t_max), 1.0f);
+    return mul(ramp, value);
+  }
+  return value;
+}
+
 // Compile-time loop: f(std::integral_constant<int, I>) for I = I0 .. N-1.
 template <int I, int N, class F>
 __device__ __forceinline__ void static_for(F&& f) {

@@ -111,16 +111,6 @@ __global__ void euler_scalar_kernel(const float* __restrict__ y, const float* __
     o[i] = add(y[i], mul(dt, k[i]));
 }
 
-// Boundary value of one group at time t (boundary_functions.py:32-45, 77-92).
-__device__ __forceinline__ float bc_value(int func, float value, float t_max, const float* t_dev) {
-  if (func == PDE_BC_FUNC_RAMP) {
-    float t = t_dev ? *t_dev : 0.0f;
-    float ramp = fminf(__fdiv_rn(t, t_max), 1.0f);
-    return mul(ramp, value);
-  }
-  return value;
-}
-
 // One boundary group, functional_boundary.py:357-400.  Reads only `in`
 // (the pre-boundary field); `out` already holds the copy of `in`.
 __global__ void bc_group_kernel(const float* __restrict__ in, float* __restrict__ out, Geo G, int N,

@@ -14,6 +14,7 @@
 #include "wave.cuh"
 #include "batched.cuh"
 #include "heat_adj.cuh"
+#include "regtile_host.h"
 
 using namespace pde;
 
@@ -647,6 +648,11 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
   const int R = W.radius;
   const bool two_d = (G.ndims == 2 && G.n[2] == 1);
   const bool s3d = !two_d && heat3d_ok(G, ncomp);
+  if (two_d && g_dispatch != PDE_DISPATCH_GENERIC && rt_heat_shape(G, ncomp, rules)) {
+    const RTPlan L = rt_heat_plan(G, nsteps, steps_per_pass, g_tile2d[0], g_tile2d[1]);
+    if (L.ok)
+      return rt_heat_run(L, u_in, u_out, work, G, W, *rules, alpha, dt, nsteps, t0, tstep, n0, st);
+  }
   int k = heat_depth(G, ncomp, steps_per_pass);
   if (k > nsteps) k = nsteps;
   if (s3d && k == 1 && heat_split_shape(G, ncomp) && aligned16(u_in) && aligned16(u_out) && aligned16(work))

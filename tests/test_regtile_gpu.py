@@ -1,0 +1,53 @@
+"""The register-tile 2D kernels against the float32 oracle, bit for bit, at the
+sizes where their windows change shape: boxes of exactly one window, one strip or
+one lane more or less, odd sides, one and several tiles per axis, both orders,
+passes that end short, every kind of face group."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import fdm
+import pde_module_b200 as P
+
+pytestmark = pytest.mark.gpu
+
+DIRICHLET = [("ALL", 1, 0.5, (0,))]
+MIXED = [("ALL", 2, 0.3, (0,)), ("-X", 1, 0.25, (0,)), ("+Y", 1, -1.0, (0,))]
+NEUMANN = [("ALL", 2, -0.4, (0,))]
+
+# interior sides (stencil box)
+SIDES = [(8, 8), (9, 11), (16, 64), (17, 65), (63, 66), (64, 64), (65, 128), (96, 129), (130, 67), (201, 333)]
+
+
+@pytest.mark.parametrize("sides", SIDES)
+@pytest.mark.parametrize("order,spec", [(2, DIRICHLET), (2, MIXED), (2, NEUMANN), (4, DIRICHLET), (4, MIXED)])
+def test_heat_rollout_window_edges(sides, order, spec):
+    g = order // 2
+    shape = (sides[0] + 2 * g, sides[1] + 2 * g, 1)
+    dx = 1.0 / sides[0]
+    dt = 0.15 * dx * dx
+    u0 = np.random.default_rng(sides[0] * 1000 + sides[1] + order).random(shape + (1,)).astype(np.float32)
+    ud = torch.from_numpy(u0).cuda()
+    bc = P.GridBoundary(ud, dx, g)
+    for name, typ, val, comps in spec:
+        bc.set_BC(name, val, typ, comps)
+    groups = fdm.standard_groups(shape, g, spec)
+    for steps, k in ((1, 0), (11, 4), (27, 0)):
+        got = P.HeatRollout(bc, dx, 0.9, dt, order=order, steps_per_pass=k)(ud, steps).cpu().numpy()
+        ref = fdm.heat_rollout(u0, groups, dx, g, 0.9, dt, steps, order)
+        assert np.array_equal(got, ref), (steps, k)
+    assert np.array_equal(ud.cpu().numpy(), u0)
+
+
+def test_heat_rollout_unfilled_ghosts_keep_the_shared_memory_path():
+    """A face no group touches keeps its ghosts' input values."""
+    shape, g = (40, 37, 1), 1
+    dx = 1.0 / 38
+    spec = [("-Y", 1, 0.4, (0,)), ("+X", 2, -0.3, (0,))]
+    u0 = np.random.default_rng(5).random(shape + (1,)).astype(np.float32)
+    ud = torch.from_numpy(u0).cuda()
+    bc = P.GridBoundary(ud, dx, g)
+    for name, typ, val, comps in spec:
+        bc.set_BC(name, val, typ, comps)
+    got = P.HeatRollout(bc, dx, 0.9, 0.15 * dx * dx)(ud, 13).cpu().numpy()
+    assert np.array_equal(got, fdm.heat_rollout(u0, fdm.standard_groups(shape, g, spec), dx, g, 0.9, 0.15 * dx * dx, 13))
