@@ -202,9 +202,9 @@ inline int sm_count() {
 // while the previous kernel of the stream runs; it calls pdl_wait before any
 // global access to data another launch reads or writes.
 template <typename... KArgs, typename... Args>
-int launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+int launch_pdl_grid(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -214,6 +214,16 @@ int launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStr
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? PDE_OK : PDE_ERR_CUDA;
+}
+
+template <typename... KArgs, typename... Args>
+int launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  return launch_pdl_grid(kern, dim3((unsigned)grid), block, smem, st, args...);
+}
+// A 2D grid without dynamic shared memory.
+template <typename... KArgs, typename... Args>
+int launch_pdl2(void (*kern)(KArgs...), dim3 grid, int block, cudaStream_t st, Args... args) {
+  return launch_pdl_grid(kern, grid, block, 0, st, args...);
 }
 
 inline int grid_blocks(int64_t work, int threads, int64_t cap = 148LL * 64) {

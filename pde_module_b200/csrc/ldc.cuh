@@ -24,32 +24,81 @@ struct LdcConst {
   float nu, dt, inv_dt, h2;
 };
 
-// The three pointwise kernels run one thread per cell on a 2D grid (row =
-// row0 + blockIdx.y; a slab of a larger domain passes its first owned row and
-// pointers shifted so that global row indices address its local rows).  A cell whose neighbours are all at least one cell inside the
-// node ring ("deep": x, y in [g+2, n-g-3]) reads raw values; the others go
-// through bc_eval2d, which returns the boundary-filled value of any cell.
-__device__ __forceinline__ bool ldc_deep(const Geo& G, int i, int j) {
-  return i >= G.g + 2 && i < (int)G.n[0] - G.g - 2 && j >= G.g + 2 && j < (int)G.n[1] - G.g - 2;
+// The predictor, divergence and projection work on shared-memory tiles: a block
+// loads its tile grown by a halo (clipped to the rows held), fills the boundary
+// there once (bc_fill_region), and every cell reads plain neighbours.  Evaluating
+// the boundary-filled value per neighbour instead, one thread per cell on global
+// memory, took 56 us a step for the three kernels on 1024^2 and 23 us on 100^2 (the
+// chain of rule look-ups of a boundary cell); these take 25 and 11.5.  Row indices are those of the whole domain; a
+// slab passes pointers shifted to them.
+constexpr int LDC_TX = 16, LDC_TY = 64, LDC_THREADS = 256;
+
+struct LdcRows {
+  int X, Y, g;
+  int own_lo, own_hi;    // rows written
+  int held_lo, held_hi;  // rows that may be read
+  bool pairs;            // the velocity arrays are 8-byte aligned
+};
+
+// Both components of a cell.
+__device__ __forceinline__ float2 ldc_ld2(const float* p, size_t cell, bool pairs) {
+  if (pairs) return reinterpret_cast<const float2*>(p)[cell];
+  return make_float2(p[2 * cell], p[2 * cell + 1]);
 }
-__device__ __forceinline__ bool ldc_stencil(const Geo& G, int i, int j) {
-  return i >= G.g && i < (int)G.n[0] - G.g && j >= G.g && j < (int)G.n[1] - G.g;
+__device__ __forceinline__ void ldc_st2(float* p, size_t cell, float2 v, bool pairs) {
+  if (pairs) {
+    reinterpret_cast<float2*>(p)[cell] = v;
+  } else {
+    p[2 * cell] = v.x;
+    p[2 * cell + 1] = v.y;
+  }
 }
 
-// Raw 2D access (ncomp N) with 32-bit cell indices.
+// Region accessor: N floats per cell, cells addressed by array indices.
 template <int N>
-struct Raw2 {
-  const float* u;
-  int n1;
-  __device__ __forceinline__ float operator()(int i, int j, int v) const { return __ldg(u + (i * n1 + j) * N + v); }
+struct Reg2 {
+  const float* s;
+  int rx0, ry0, RY;
+  __device__ __forceinline__ float operator()(int i, int j, int v) const {
+    return s[((i - rx0) * RY + (j - ry0)) * N + v];
+  }
 };
-// Boundary-filled access.
-struct Bc2 {
-  const Geo& G;
-  const PdeBCRules& R;
-  const GlobalAcc& U;
-  __device__ __forceinline__ float operator()(int i, int j, int v) const { return bc_eval2d(G, R, U, i, j, v); }
+
+// A block's tile and region (tile + halo, within the array and the held rows).
+struct LdcTile {
+  int bx0, by0, bx1, by1, rx0, ry0, RX, RY;
+  __device__ LdcTile(const LdcRows& D, int halo) {
+    bx0 = D.own_lo + (int)blockIdx.y * LDC_TX;
+    by0 = (int)blockIdx.x * LDC_TY;
+    bx1 = min(bx0 + LDC_TX, D.own_hi);
+    by1 = min(by0 + LDC_TY, D.Y);
+    rx0 = max(bx0 - halo, D.held_lo);
+    ry0 = max(by0 - halo, 0);
+    RX = min(bx1 + halo, D.held_hi) - rx0;
+    RY = min(by1 + halo, D.Y) - ry0;
+  }
+  // fn(region index, x, y) over the region's cells / the tile's cells
+  template <class F>
+  __device__ __forceinline__ void region(F fn) const {
+    RectWalk wk(RY, LDC_THREADS);
+    for (int i = threadIdx.x; i < RX * RY; i += LDC_THREADS, wk.next()) fn(i, rx0 + wk.row, ry0 + wk.col);
+  }
+  template <class F>
+  __device__ __forceinline__ void tile(F fn) const {
+    const int W = by1 - by0, n = (bx1 - bx0) * W;
+    RectWalk wk(W, LDC_THREADS);
+    for (int i = threadIdx.x; i < n; i += LDC_THREADS, wk.next()) fn(bx0 + wk.row, by0 + wk.col);
+  }
 };
+
+__device__ __forceinline__ bool ldc_stencil(const LdcRows& D, int i, int j) {
+  return i >= D.g && i < D.X - D.g && j >= D.g && j < D.Y - D.g;
+}
+__device__ __forceinline__ H2Params ldc_shape(const LdcRows& D) {
+  H2Params H;
+  H.X = D.X; H.Y = D.Y; H.g = D.g; H.N = 1;
+  return H;
+}
 
 // Predictor of one stencil cell: u* = u2 + dt * (nu*Lap(u2) - Grad(u2) u2), with u2 = BC_u(u).
 template <class Get>
@@ -86,25 +135,6 @@ __device__ __forceinline__ void ldc_predict_cell(const Get& at, int i, int j, co
   }
 }
 
-__global__ void __launch_bounds__(256) ldc_predictor_kernel(const float* __restrict__ u, float* __restrict__ us,
-                                                             Geo G, const PdeBCRules Ru, LdcConst K, int row0) {
-  const int i = row0 + (int)blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (int)G.n[1]) return;
-  const int n1 = (int)G.n[1];
-  const int cell = i * n1 + j;
-  GlobalAcc U{u, G.cstride[0], G.cstride[1], 2};
-  if (!ldc_stencil(G, i, j)) {
-    us[cell * 2 + 0] = bc_eval2d(G, Ru, U, i, j, 0);
-    us[cell * 2 + 1] = bc_eval2d(G, Ru, U, i, j, 1);
-    return;
-  }
-  float res[2];
-  if (ldc_deep(G, i, j)) ldc_predict_cell(Raw2<2>{u, n1}, i, j, K, res);
-  else ldc_predict_cell(Bc2{G, Ru, U}, i, j, K, res);
-  us[cell * 2 + 0] = res[0];
-  us[cell * 2 + 1] = res[1];
-}
-
 // rhs = (1/dt) * Div(BC_u(u*)) on stencil cells (ghosts of rhs are never read).
 template <class Get>
 __device__ __forceinline__ float ldc_div_cell(const Get& at, int i, int j, const LdcConst& K) {
@@ -116,18 +146,57 @@ __device__ __forceinline__ float ldc_div_cell(const Get& at, int i, int j, const
   return mul(K.inv_dt, acc);
 }
 
-__global__ void __launch_bounds__(256) ldc_divergence_kernel(const float* __restrict__ us, float* __restrict__ rhs,
-                                                              Geo G, const PdeBCRules Ru, LdcConst K, int row0) {
-  const int i = row0 + (int)blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (int)G.n[1]) return;
-  const int n1 = (int)G.n[1];
-  const int cell = i * n1 + j;
-  if (!ldc_stencil(G, i, j)) {
-    rhs[cell] = 0.0f;
-    return;
+// PREDICT: u -> u*.  DIVERGE: u* -> rhs.  Both: u* of the tile and one cell around it
+// stays in shared memory for the divergence (a slab runs them one by one: u* rows
+// of the neighbouring slab come between).
+template <bool PREDICT, bool DIVERGE>
+__global__ void __launch_bounds__(LDC_THREADS) ldc_velocity_kernel(const float* __restrict__ u, float* us,
+                                                                   float* __restrict__ rhs, const LdcRows D,
+                                                                   const PdeBCRules Ru, const LdcConst K) {
+  pdl_launch_dependents();
+  constexpr int HALO = PREDICT && DIVERGE ? 2 : 1;
+  constexpr int CAP = (LDC_TX + 2 * HALO) * (LDC_TY + 2 * HALO);
+  __shared__ float2 A[PREDICT ? CAP : 1], B[DIVERGE ? CAP : 1];
+  const LdcTile T(D, HALO);
+  const H2Params HP = ldc_shape(D);
+  pdl_wait();
+  const float* src = PREDICT ? u : us;
+  float2* first = PREDICT ? A : B;
+  T.region([&](int i, int x, int y) { first[i] = ldc_ld2(src, (size_t)x * D.Y + y, D.pairs); });
+  __syncthreads();
+  if constexpr (PREDICT) {
+    bc_fill_region<2>(reinterpret_cast<float*>(A), HP, Ru, T.rx0, T.RX, T.ry0, T.RY, Ru.dx32);
+    __syncthreads();
+    const Reg2<2> at{reinterpret_cast<const float*>(A), T.rx0, T.ry0, T.RY};
+    auto value = [&](int x, int y) {
+      float res[2] = {at(x, y, 0), at(x, y, 1)};
+      if (ldc_stencil(D, x, y)) ldc_predict_cell(at, x, y, K, res);
+      return make_float2(res[0], res[1]);
+    };
+    if constexpr (!DIVERGE) {
+      T.tile([&](int x, int y) { ldc_st2(us, (size_t)x * D.Y + y, value(x, y), D.pairs); });
+      return;
+    } else {
+      T.region([&](int i, int x, int y) {
+        // the region's outer ring has no complete neighbourhood and is not read
+        const bool ring = (x == T.rx0 && x > 0) || (x == T.rx0 + T.RX - 1 && x < D.X - 1) || (y == T.ry0 && y > 0) ||
+                          (y == T.ry0 + T.RY - 1 && y < D.Y - 1);
+        const float2 v = ring ? A[i] : value(x, y);
+        B[i] = v;
+        if (x >= T.bx0 && x < T.bx1 && y >= T.by0 && y < T.by1)
+          ldc_st2(us, (size_t)x * D.Y + y, v, D.pairs);
+      });
+      __syncthreads();
+    }
   }
-  GlobalAcc U{us, G.cstride[0], G.cstride[1], 2};
-  rhs[cell] = ldc_deep(G, i, j) ? ldc_div_cell(Raw2<2>{us, n1}, i, j, K) : ldc_div_cell(Bc2{G, Ru, U}, i, j, K);
+  if constexpr (DIVERGE) {
+    bc_fill_region<2>(reinterpret_cast<float*>(B), HP, Ru, T.rx0, T.RX, T.ry0, T.RY, Ru.dx32);
+    __syncthreads();
+    const Reg2<2> at{reinterpret_cast<const float*>(B), T.rx0, T.ry0, T.RY};
+    T.tile([&](int x, int y) {
+      rhs[(size_t)x * D.Y + y] = ldc_stencil(D, x, y) ? ldc_div_cell(at, x, y, K) : 0.0f;
+    });
+  }
 }
 
 // u = BC_u(u*) + dt * Grad(BC_p(p), -1)
@@ -144,25 +213,33 @@ __device__ __forceinline__ void ldc_project_cell(const GetU& au, const GetP& ap,
   res[1] = add(a1, mul(K.dt, mul(-1.0f, gy)));
 }
 
-__global__ void __launch_bounds__(256) ldc_project_kernel(const float* __restrict__ us, const float* __restrict__ p,
-                                                           float* __restrict__ u, Geo G, const PdeBCRules Ru,
-                                                           const PdeBCRules Rp, LdcConst K, int row0) {
-  const int i = row0 + (int)blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= (int)G.n[1]) return;
-  const int n1 = (int)G.n[1];
-  const int cell = i * n1 + j;
-  GlobalAcc U{us, G.cstride[0], G.cstride[1], 2};
-  GlobalAcc Pa{p, G.cstride[0], G.cstride[1], 1};
-  if (!ldc_stencil(G, i, j)) {
-    u[cell * 2 + 0] = bc_eval2d(G, Ru, U, i, j, 0);
-    u[cell * 2 + 1] = bc_eval2d(G, Ru, U, i, j, 1);
-    return;
-  }
-  float res[2];
-  if (ldc_deep(G, i, j)) ldc_project_cell(Raw2<2>{us, n1}, Raw2<1>{p, n1}, i, j, K, res);
-  else ldc_project_cell(Bc2{G, Ru, U}, Bc2{G, Rp, Pa}, i, j, K, res);
-  u[cell * 2 + 0] = res[0];
-  u[cell * 2 + 1] = res[1];
+__global__ void __launch_bounds__(LDC_THREADS) ldc_project_kernel(const float* __restrict__ us,
+                                                                   const float* __restrict__ p, float* __restrict__ u,
+                                                                   const LdcRows D, const PdeBCRules Ru,
+                                                                   const PdeBCRules Rp, const LdcConst K) {
+  pdl_launch_dependents();
+  constexpr int CAP = (LDC_TX + 2) * (LDC_TY + 2);
+  __shared__ float2 A[CAP];
+  __shared__ float Pr[CAP];
+  const LdcTile T(D, 1);
+  const H2Params HP = ldc_shape(D);
+  pdl_wait();
+  T.region([&](int i, int x, int y) {
+    const size_t c = (size_t)x * D.Y + y;
+    A[i] = ldc_ld2(us, c, D.pairs);
+    Pr[i] = p[c];
+  });
+  __syncthreads();
+  bc_fill_region<2>(reinterpret_cast<float*>(A), HP, Ru, T.rx0, T.RX, T.ry0, T.RY, Ru.dx32);
+  bc_fill_region<1>(Pr, HP, Rp, T.rx0, T.RX, T.ry0, T.RY, Rp.dx32);
+  __syncthreads();
+  const Reg2<2> au{reinterpret_cast<const float*>(A), T.rx0, T.ry0, T.RY};
+  const Reg2<1> ap{Pr, T.rx0, T.ry0, T.RY};
+  T.tile([&](int x, int y) {
+    float res[2] = {au(x, y, 0), au(x, y, 1)};
+    if (ldc_stencil(D, x, y)) ldc_project_cell(au, ap, x, y, K, res);
+    ldc_st2(u, (size_t)x * D.Y + y, make_float2(res[0], res[1]), D.pairs);
+  });
 }
 
 // k Jacobi sweeps per pass on shared-memory tiles (halo k + 1, as in
@@ -259,127 +336,6 @@ __global__ void __launch_bounds__(1024) jacobi2d_tb_kernel(const float* __restri
     const int ri = (x - rx0) * RY + (y - ry0);
     const bool st = x >= g && x < P.X - g && y >= g && y < P.Y - g;
     pout[(size_t)x * P.Y + y] = st ? A[ri] : B[ri];  // (equal when k = 0: both hold the loaded values)
-  }
-  if (P.last && resid) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    __shared__ float wsum[32];
-    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = sq;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float b = 0.0f;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b += wsum[w];
-      atomicAdd(resid, b);
-    }
-  }
-}
-
-// The same passes with register cell lists (as the wave kernels): the region's
-// cells interleave the two levels and the right-hand side (3 floats per cell, an
-// odd stride: no bank conflicts), each thread's stencil cells are fixed for the
-// pass (slots q = threadIdx.x + c * blockDim.x over the stencil rectangle's rows
-// at full region width, the columns outside the rectangle idle), with their
-// region index and distance from the tile (one packed word: index in the low 16
-// bits, regions hold fewer than 2^16 cells) and h^2 rhs in registers (h^2 rhs is
-// the same product every sweep).  Sweep s reads level s & 1 and writes the other;
-// two sweeps per loop iteration make the levels compile-time offsets.  Same
-// arithmetic and order per cell as jacobi2d_tb_kernel; needs the rectangle's
-// rows x RY <= MAXC * blockDim.x.
-template <int MAXC>
-__global__ void __launch_bounds__(1024) jacobi2d_cells_kernel(const float* __restrict__ pin,
-                                                              float* __restrict__ pout,
-                                                              const float* __restrict__ rhs,
-                                                              float* __restrict__ resid, const J2Params P,
-                                                              const PdeBCRules Rp) {
-  pdl_launch_dependents();  // the next pass may be scheduled; it waits for this one
-  extern __shared__ __align__(16) float sm[];
-  constexpr int NB = 3;  // per region cell: level 0, level 1, rhs
-  const int tx = blockIdx.x / P.tiles_y, ty = blockIdx.x % P.tiles_y;
-  const int bx0 = P.own_lo + tx * P.TBX, by0 = ty * P.TBY;
-  const int H = P.k + 1;
-  const int rx0 = max(bx0 - H, P.held_lo), rx1 = min(bx0 + P.TBX + H, P.held_hi);
-  const int ry0 = max(by0 - H, 0), ry1 = min(by0 + P.TBY + H, P.Y);
-  const int RX = rx1 - rx0, RY = ry1 - ry0, RC = RX * RY;
-  const int nt = (int)blockDim.x;
-  H2Params HP;
-  HP.X = P.X; HP.Y = P.Y; HP.g = P.g; HP.N = 1;
-  const int g = P.g;
-  // stencil rectangle: cells of [g, n-g) whose four neighbours are inside the region
-  const int sx0 = max(g, rx0 + 1) - rx0, sx1 = min(P.X - g, rx0 + RX - 1) - rx0;
-  const int sy0 = max(g, ry0 + 1) - ry0, sy1 = min(P.Y - g, ry0 + RY - 1) - ry0;
-  const int tw = min(bx0 + P.TBX, P.own_hi) - bx0, th = min(by0 + P.TBY, P.Y) - by0;
-  const int tlx = bx0 - rx0, tly = by0 - ry0;  // the tile's origin in the region
-  int key[MAXC];  // region index | distance from the tile << 16; idle slots: INT_MAX
-  float hr[MAXC];
-  unsigned tile = 0;  // bit c: slot c holds a tile cell (residual)
-  {
-    const int n = max(sx1 - sx0, 0) * RY;
-    RectWalk wk(RY, nt);
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      key[c] = 0x7fffffff;
-      if ((int)threadIdx.x + c * nt < n && wk.col >= sy0 && wk.col < sy1) {
-        const int lx = sx0 + wk.row, ly = wk.col;
-        const int ox = lx - tlx, oy = ly - tly;
-        const int d = max(max(max(-ox, ox - (tw - 1)), max(-oy, oy - (th - 1))), 0);
-        key[c] = (lx * RY + ly) | (d << 16);
-        if (ox >= 0 && ox < tw && oy >= 0 && oy < th) tile |= 1u << c;
-      }
-      wk.next();
-    }
-  }
-  const int rs = NB * RY;
-  float sq = 0.0f;
-  BcPlan<1> bp;
-  bc_plan(bp, HP, rx0, RX, ry0, RY);
-  pdl_wait();  // the previous pass's pressure (this pass's input) is complete
-  {
-    RectWalk wk(RY, nt);
-    for (int i = threadIdx.x; i < RC; i += nt, wk.next()) {
-      const size_t gi = (size_t)(rx0 + wk.row) * P.Y + ry0 + wk.col;
-      cp_async4(sm + NB * i, pin + gi, true);
-      cp_async4(sm + NB * i + 1, pin + gi, true);
-      cp_async4(sm + NB * i + 2, rhs + gi, true);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-#pragma unroll
-  for (int c = 0; c < MAXC; ++c)  // h^2 rhs of the thread's cells (the same product every sweep)
-    hr[c] = key[c] != 0x7fffffff ? mul(P.h2, sm[NB * (key[c] & 0xffff) + 2]) : 0.0f;
-  // Sweep s only has to update the stencil cells within (k - 1 - s) + 1 of the
-  // tile (the boundary fills read inward): those with dist <= k - s.
-  auto sweep = [&](auto PAR, int s) {
-    constexpr int p = decltype(PAR)::value;  // reads level p, writes level 1 - p
-    bc_fill_planned<1, NB>(sm + p, bp, HP, Rp, rx0, RX, ry0, RY, Rp.dx32);
-    const bool acc_res = P.last && s == P.k - 1;
-    const int lim = (P.k - s + 1) << 16;  // dist <= k - s  <=>  key < lim
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      if (key[c] >= lim) continue;
-      float* pc = sm + NB * (key[c] & 0xffff);
-      const float sum = add(add(add(pc[p - rs], pc[p + rs]), pc[p - NB]), pc[p + NB]);
-      const float res = mul(0.25f, sub(sum, hr[c]));
-      if (acc_res && ((tile >> c) & 1u)) {
-        const float d = res - pc[p];
-        sq = fmaf(d, d, sq);
-      }
-      pc[1 - p] = res;
-    }
-    __syncthreads();
-  };
-  for (int s = 0; s < P.k; s += 2) {
-    sweep(std::integral_constant<int, 0>{}, s);
-    if (s + 1 < P.k) sweep(std::integral_constant<int, 1>{}, s + 1);
-  }
-  // output: stencil cells from the newest level, the others as last filled
-  const int nw = P.k & 1;  // the level the last sweep wrote
-  RectWalk wo(th, nt);
-  for (int i = threadIdx.x; i < tw * th; i += nt, wo.next()) {
-    const int x = bx0 + wo.row, y = by0 + wo.col;
-    const int r = (x - rx0) * RY + (y - ry0);
-    const bool st = x >= g && x < P.X - g && y >= g && y < P.Y - g;
-    pout[(size_t)x * P.Y + y] = sm[NB * r + (st ? nw : 1 - nw)];
   }
   if (P.last && resid) {
 #pragma unroll

@@ -1254,72 +1254,55 @@ int ldc_setup(const PdeGrid* grid, const PdeBCRules* u_rules, const PdeBCRules* 
   return PDE_OK;
 }
 
-// Jacobi launch geometry for k sweeps per pass over owned rows [own_lo, own_hi)
-// of arrays holding rows [held_lo, held_hi) of a domain of G.n[0] rows.
+// Jacobi sweeps over owned rows [own_lo, own_hi) of arrays holding rows
+// [held_lo, held_hi) of a domain of G.n[0] rows: register tiles, or the
+// shared-memory kernel for the shapes and rules those do not take (boxes under 8
+// cells a side, faces no pressure group fills, tiles set too large for a window).
 struct JacobiLaunch {
-  int tiles, threads, cpt;  // cpt: register cells per thread (0: the flat-walk kernel)
+  RTPlan rt;
+  JacobiRun run;
+  J2Params JP;
+  int tiles, threads, k;
   size_t smem;
 };
 
-int jacobi_setup(const Geo& G, float h2, int k, int own_lo, int own_hi, int held_lo, int held_hi, J2Params* JP,
-                 JacobiLaunch* L) {
+// k: deepest pass, only: exactly that depth (a slab's halo is exchanged per pass).
+int jacobi_setup(const Geo& G, float h2, int nsweeps, int k, bool only, int own_lo, int own_hi, int held_lo, int held_hi,
+                 const PdeBCRules& rules, JacobiLaunch* L) {
+  L->run = JacobiRun{(int)G.n[0], (int)G.n[1], G.g, own_lo, own_hi, held_lo, held_hi, h2};
+  L->rt.ok = false;
+  if (rt_fills_all_faces(rules)) L->rt = rt_jacobi_plan(L->run, nsweeps, k, only, g_tile2d[0], g_tile2d[1]);
+  if (L->rt.ok) {
+    L->k = L->rt.k;
+    return PDE_OK;
+  }
+  L->k = k > 0 ? k : 10;
+  if (L->k > nsweeps && nsweeps > 0) L->k = nsweeps;
+  J2Params* JP = &L->JP;
   JP->X = (int)G.n[0]; JP->Y = (int)G.n[1]; JP->g = G.g;
   JP->own_lo = own_lo; JP->own_hi = own_hi; JP->held_lo = held_lo; JP->held_hi = held_hi;
-  bool placed = false;
-  if (g_tile2d[0] == 0 && g_threads2d == 0) {
-    // automatic shape on grids that fill the SMs: one near-square tile per SM,
-    // 1024 threads (the register cell-list kernel, at most 12 cells per thread)
-    const int rows = own_hi - own_lo, sms = (int)sm_count();
-    int nx = (int)lround(sqrt((double)sms * rows / JP->Y));
-    nx = nx < 1 ? 1 : (nx > sms ? sms : nx);
-    const int ny = sms / nx > 0 ? sms / nx : 1;
-    const int tx = (rows + nx - 1) / nx, ty = (JP->Y + ny - 1) / ny;
-    const long long capb = (long long)(tx + 2 * (k + 1)) * (ty + 2 * (k + 1));
-    if (tx >= 32 && ty >= 32 && tx <= 256 && ty <= 256 && capb <= 12LL * 1024 && capb < (1 << 16)) {
-      JP->TBX = tx;
-      JP->TBY = ty;
-      L->threads = 1024;
-      placed = true;
-    }
-  }
-  if (!placed) {
-    pick_tile_2d(JP->X, JP->Y, &JP->TBX, &JP->TBY);
-    L->threads = g_threads2d > 0 ? g_threads2d : 256;
-  }
+  pick_tile_2d(JP->X, JP->Y, &JP->TBX, &JP->TBY);
+  L->threads = g_threads2d > 0 ? g_threads2d : 256;
   JP->tiles_y = (JP->Y + JP->TBY - 1) / JP->TBY;
-  JP->RXM = JP->TBX + 2 * (k + 1);
-  JP->RYM = JP->TBY + 2 * (k + 1);
+  JP->RXM = JP->TBX + 2 * (L->k + 1);
+  JP->RYM = JP->TBY + 2 * (L->k + 1);
   JP->h2 = h2;
   L->tiles = ((own_hi - own_lo + JP->TBX - 1) / JP->TBX) * JP->tiles_y;
-  // the register cell lists cover every block's stencil rows x RY <= RXM x RYM
-  const long long cap = (long long)JP->RXM * JP->RYM;
-  L->cpt = cap <= 4LL * L->threads ? 4 : cap <= 6LL * L->threads ? 6 : cap <= 8LL * L->threads ? 8
-         : cap <= 12LL * L->threads ? 12 : 0;
-  L->smem = (size_t)3 * cap * sizeof(float);  // both kernels: two levels and the rhs per cell
+  L->smem = (size_t)3 * JP->RXM * JP->RYM * sizeof(float);  // two levels and the rhs per cell
   if (L->smem > 227 * 1024) return PDE_ERR_TOO_LARGE;
-  if (cap >= (1 << 16)) L->cpt = 0;  // the cell lists pack region indices in 16 bits
-  const void* kern = L->cpt == 4 ? (const void*)jacobi2d_cells_kernel<4>
-                   : L->cpt == 6 ? (const void*)jacobi2d_cells_kernel<6>
-                   : L->cpt == 8 ? (const void*)jacobi2d_cells_kernel<8>
-                   : L->cpt == 12 ? (const void*)jacobi2d_cells_kernel<12>
-                                  : (const void*)jacobi2d_tb_kernel;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) != cudaSuccess)
+  if (cudaFuncSetAttribute((const void*)jacobi2d_tb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) !=
+      cudaSuccess)
     return PDE_ERR_CUDA;
   return PDE_OK;
 }
 
-int launch_jacobi(const JacobiLaunch& L, cudaStream_t st, const float* pin, float* pout, const float* rhs,
-                  float* resid, const J2Params& JP, const PdeBCRules& R) {
-  switch (L.cpt) {
-    case 4: return launch_pdl(jacobi2d_cells_kernel<4>, L.tiles, L.threads, L.smem, st, pin, pout, rhs, resid, JP, R);
-    case 6: return launch_pdl(jacobi2d_cells_kernel<6>, L.tiles, L.threads, L.smem, st, pin, pout, rhs, resid, JP, R);
-    case 8: return launch_pdl(jacobi2d_cells_kernel<8>, L.tiles, L.threads, L.smem, st, pin, pout, rhs, resid, JP, R);
-    case 12:
-      return launch_pdl(jacobi2d_cells_kernel<12>, L.tiles, L.threads, L.smem, st, pin, pout, rhs, resid, JP, R);
-    default:
-      jacobi2d_tb_kernel<<<L.tiles, L.threads, L.smem, st>>>(pin, pout, rhs, resid, JP, R);
-      return launch_status();
-  }
+int launch_jacobi(JacobiLaunch& L, int k, bool last, cudaStream_t st, const float* pin, float* pout, const float* rhs,
+                  float* resid, const PdeBCRules& R) {
+  if (L.rt.ok) return rt_jacobi_pass(L.rt, L.run, pin, pout, rhs, resid, k, last, R, st);
+  L.JP.k = k;
+  L.JP.last = last ? 1 : 0;
+  jacobi2d_tb_kernel<<<L.tiles, L.threads, L.smem, st>>>(pin, pout, rhs, resid, L.JP, R);
+  return launch_status();
 }
 
 }  // namespace
@@ -1346,37 +1329,35 @@ int ldc_rollout_run(float* u, float* p, float* u_star, float* p_tmp, float* rhs,
   cudaStream_t st = as_stream(stream);
   const int64_t cells = G.n[0] * G.n[1];
   const int X = (int)G.n[0];
-  const dim3 grid2((unsigned)((G.n[1] + 255) / 256), (unsigned)X);
+  const bool pairs = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(u_star)) & 7u) == 0;
+  const LdcRows D{X, (int)G.n[1], G.g, 0, X, 0, X, pairs};
+  const dim3 tiles((unsigned)((D.Y + LDC_TY - 1) / LDC_TY), (unsigned)((X + LDC_TX - 1) / LDC_TX));
   if (resid && nsteps > 0) PDE_CUDA_CHECK(cudaMemsetAsync(resid, 0, sizeof(float) * nsteps, st));
   const int iters = prm->jacobi_iters;
-  int k = prm->jacobi_per_pass > 0 ? prm->jacobi_per_pass : 10;
-  if (k > iters && iters > 0) k = iters;
-  J2Params JP;
   JacobiLaunch JL;
-  rc = jacobi_setup(G, K.h2, k, 0, X, 0, X, &JP, &JL);
+  rc = jacobi_setup(G, K.h2, iters, prm->jacobi_per_pass, false, 0, X, 0, X, *p_rules_in, &JL);
   if (rc) return rc;
+  const int npasses = JL.k > 0 ? (iters + JL.k - 1) / JL.k : 0;
   for (int step = 0; step < nsteps; ++step) {
     // time-dependent groups: step n fills every boundary at t0 + n * tstep
     const PdeBCRules ur = rules_at(*u_rules_in, t0, tstep, step), pr = rules_at(*p_rules_in, t0, tstep, step);
     const PdeBCRules* u_rules = &ur;
     const PdeBCRules* p_rules = &pr;
-    ldc_predictor_kernel<<<grid2, 256, 0, st>>>(u, u_star, G, *u_rules, K, 0);
-    ldc_divergence_kernel<<<grid2, 256, 0, st>>>(u_star, rhs, G, *u_rules, K, 0);
+    rc = launch_pdl2(ldc_velocity_kernel<true, true>, tiles, LDC_THREADS, st, u, u_star, rhs, D, *u_rules, K);
+    if (rc) return rc;
     float* src = p;
     float* dst = p_tmp;
-    for (int done = 0; done < iters;) {
-      JP.k = (iters - done < k) ? (iters - done) : k;
-      done += JP.k;
-      JP.last = (done == iters);
-      rc = launch_jacobi(JL, st, src, dst, rhs, resid ? resid + step : nullptr, JP, *p_rules);
+    for (int pass = 0, done = 0; done < iters; ++pass) {
+      const int ks = (iters - done + npasses - pass - 1) / (npasses - pass);  // passes of even depth
+      done += ks;
+      rc = launch_jacobi(JL, ks, done == iters, st, src, dst, rhs, resid ? resid + step : nullptr, *p_rules);
       if (rc) return rc;
       float* t = src;
       src = dst;
       dst = t;
     }
     if (src != p) PDE_CUDA_CHECK(cudaMemcpyAsync(p, src, sizeof(float) * cells, cudaMemcpyDeviceToDevice, st));
-    ldc_project_kernel<<<grid2, 256, 0, st>>>(u_star, p, u, G, *u_rules, *p_rules, K, 0);
-    rc = launch_status();
+    rc = launch_pdl2(ldc_project_kernel, tiles, LDC_THREADS, st, u_star, p, u, D, *u_rules, *p_rules, K);
     if (rc) return rc;
   }
   return PDE_OK;
@@ -1496,7 +1477,9 @@ int pde_ldc_slab_step(int32_t phase, float* u, float* u_star, const float* p_in,
   cudaStream_t st = as_stream(stream);
   // pointers addressed by global row: local row r is global row off + r
   auto gl = [&](const float* q, int ncomp) { return q ? q - off * Y * ncomp : nullptr; };
-  const dim3 grid2((unsigned)((Y + 255) / 256), (unsigned)(hi - lo));
+  const LdcRows D{(int)Xg, (int)Y, G.g, (int)lo, (int)hi, (int)off, (int)(off + nloc),
+                  ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(u_star)) & 7u) == 0};
+  const dim3 tiles((unsigned)((Y + LDC_TY - 1) / LDC_TY), (unsigned)((hi - lo + LDC_TX - 1) / LDC_TX));
   // rows one beyond the owned range on a cut side must be held (halo)
   const bool cut_lo = lo > 0, cut_hi = hi < Xg;
   // a ghost row's fill reads the row two steps inward: a slab with a physical
@@ -1508,30 +1491,31 @@ int pde_ldc_slab_step(int32_t phase, float* u, float* u_star, const float* p_in,
   switch (phase) {
     case PDE_LDC_PREDICT:
       if (!u || !u_star) return PDE_ERR_ARG;
-      ldc_predictor_kernel<<<grid2, 256, 0, st>>>(gl(u, 2), const_cast<float*>(gl(u_star, 2)), G, *u_rules, K,
-                                                  (int)lo);
+      rc = launch_pdl2(ldc_velocity_kernel<true, false>, tiles, LDC_THREADS, st, gl(u, 2),
+                       const_cast<float*>(gl(u_star, 2)), static_cast<float*>(nullptr), D, *u_rules, K);
+      if (rc) return rc;
       break;
     case PDE_LDC_DIVERGENCE:
       if (!u_star || !rhs) return PDE_ERR_ARG;
-      ldc_divergence_kernel<<<grid2, 256, 0, st>>>(gl(u_star, 2), const_cast<float*>(gl(rhs, 1)), G, *u_rules, K,
-                                                   (int)lo);
+      rc = launch_pdl2(ldc_velocity_kernel<false, true>, tiles, LDC_THREADS, st, static_cast<const float*>(nullptr),
+                       const_cast<float*>(gl(u_star, 2)), const_cast<float*>(gl(rhs, 1)), D, *u_rules, K);
+      if (rc) return rc;
       break;
     case PDE_LDC_PROJECT:
       if (!u || !u_star || !p_in) return PDE_ERR_ARG;
-      ldc_project_kernel<<<grid2, 256, 0, st>>>(gl(u_star, 2), gl(p_in, 1), const_cast<float*>(gl(u, 2)), G,
-                                                *u_rules, *p_rules, K, (int)lo);
+      rc = launch_pdl2(ldc_project_kernel, tiles, LDC_THREADS, st, gl(u_star, 2), gl(p_in, 1),
+                       const_cast<float*>(gl(u, 2)), D, *u_rules, *p_rules, K);
+      if (rc) return rc;
       break;
     case PDE_LDC_JACOBI: {
       if (!p_in || !p_out || !rhs || nsweeps < 1 || p_in == p_out) return PDE_ERR_ARG;
       // k sweeps invalidate k + 1 rows inward from a cut side of the held rows
       if ((cut_lo && lo - (nsweeps + 1) < off) || (cut_hi && hi + nsweeps + 1 > off + nloc)) return PDE_ERR_SHAPE;
-      J2Params JP;
       JacobiLaunch JL;
-      rc = jacobi_setup(G, K.h2, nsweeps, (int)lo, (int)hi, (int)off, (int)(off + nloc), &JP, &JL);
+      rc = jacobi_setup(G, K.h2, nsweeps, nsweeps, true, (int)lo, (int)hi, (int)off, (int)(off + nloc), *p_rules, &JL);
       if (rc) return rc;
-      JP.k = nsweeps;
-      JP.last = last ? 1 : 0;
-      rc = launch_jacobi(JL, st, gl(p_in, 1), const_cast<float*>(gl(p_out, 1)), gl(rhs, 1), resid, JP, *p_rules);
+      rc = launch_jacobi(JL, nsweeps, last != 0, st, gl(p_in, 1), const_cast<float*>(gl(p_out, 1)), gl(rhs, 1), resid,
+                         *p_rules);
       if (rc) return rc;
       break;
     }

@@ -13,10 +13,11 @@ namespace {
 
 // Window and tile along one axis for nt tiles: the rows (columns) the window
 // needs, a multiple of `unit` and at most n, or 0 when it does not fit in `cap`.
-int axis_window(int n, int nt, int H, int unit, int cap) {
+// `hold`: the cells the window may use; n < hold (a slab's rows): halo on both sides.
+int axis_window(int n, int hold, int nt, int H, int unit, int cap) {
   const int tile = (n + nt - 1) / nt;
-  const int most = n / unit * unit;
-  const int need = nt == 1 ? n : nt == 2 ? tile + H : tile + 2 * H;
+  const int most = hold / unit * unit;
+  const int need = n < hold ? tile + 2 * H : nt == 1 ? n : nt == 2 ? tile + H : tile + 2 * H;
   int win = (need + unit - 1) / unit * unit;
   if (win > most) win = most;
   if (win < need || win > cap || (long long)(nt - 1) * tile >= n) return 0;
@@ -32,13 +33,15 @@ int axis_window(int n, int nt, int H, int unit, int cap) {
 // share of that rate the kernels reach) or, when there is little of it, the
 // latency of publish, barrier, read and the dependent sums; a pass of k steps costs
 // a dependent launch and the loads and stores of its windows.
-RTPlan rt_plan(const RTCost& cost, int X, int Y, int R, int nsteps, int k_req, int tile_x, int tile_y, int sms) {
+RTPlan rt_plan(const RTCost& cost, int BX, int Y, int X0, int X1, int R, int nsteps, int k_req, bool k_only,
+               int tile_x, int tile_y, int sms) {
+  const int X = X1 - X0;
   RTPlan best;
   best.ok = false;
   best.cycles = 1e30;
   auto consider = [&](int ci, int C, int RPT, int k, int nx, int ny) {
     const int H = k * R;
-    const int nr = axis_window(X, nx, H, RPT, rt_max_warps(C, RPT) * RPT), nc = axis_window(Y, ny, H, C, 32 * C);
+    const int nr = axis_window(X, BX, nx, H, RPT, cost.max_warps[ci] * RPT), nc = axis_window(Y, Y, ny, H, C, 32 * C);
     if (nr < 2 * RPT || nc < 2 * C) return;
     const long long tiles = (long long)nx * ny;
     const int tbx = (X + nx - 1) / nx, tby = (Y + ny - 1) / ny;
@@ -55,32 +58,33 @@ RTPlan rt_plan(const RTCost& cost, int X, int Y, int R, int nsteps, int k_req, i
     best.C = C;
     best.RPT = RPT;
     best.k = k;
-    best.W = RTGeom{X, Y, tbx, tby, ny, H, nr, nc};
+    best.W = RTGeom{BX, Y, X0, X1, true, true, tbx, tby, ny, H, nr, nc};
     best.tiles = (int)tiles;
     best.threads = nr / RPT * 32;
   };
   // fewest tiles along an axis of n whose windows of at most cap hold tile and halo
-  auto fewest = [](int n, int H, int unit, int cap) {
-    if (n <= cap && n % unit == 0) return 1;
+  auto fewest = [](int n, int hold, int H, int unit, int cap) {
+    if (n == hold && n <= cap && n % unit == 0) return 1;
     const int two = (n + 1) / 2 + H;
-    if (two <= cap / unit * unit && two <= n / unit * unit) return 2;
+    if (n == hold && two <= cap / unit * unit && two <= n / unit * unit) return 2;
     const int room = cap / unit * unit - 2 * H;
     return room < 1 ? 0 : (n + room - 1) / room;
   };
-  static const int depths[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24};
+  static const int depths[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 17, 20, 24, 25};
   for (int ci = 0; ci < 4; ++ci) {
     if (!((cost.shapes >> ci) & 1)) continue;
     const int C = ci & 1 ? 4 : 2, RPT = ci & 2 ? 8 : 4;
-    for (int k : depths) {
+    for (int d : depths) {
+      const int k = k_only ? k_req : d;
       if (k > nsteps || (k_req > 0 && k > k_req)) break;
-      int ny = tile_y > 0 ? (Y + tile_y - 1) / tile_y : fewest(Y, k * R, C, 32 * C);
+      int ny = tile_y > 0 ? (Y + tile_y - 1) / tile_y : fewest(Y, Y, k * R, C, 32 * C);
       if (ny < 1) break;
       for (int more = 0; more < 3; ++more, ++ny) {
         if (tile_x > 0) {
           consider(ci, C, RPT, k, (X + tile_x - 1) / tile_x, ny);
         } else {
           // the largest windows, and as many tiles as fill the SMs once or twice
-          const int lo = fewest(X, k * R, RPT, rt_max_warps(C, RPT) * RPT);
+          const int lo = fewest(X, BX, k * R, RPT, cost.max_warps[ci] * RPT);
           if (lo < 1) break;
           consider(ci, C, RPT, k, lo, ny);
           for (int m = 1; m <= 2; ++m) {
@@ -90,6 +94,7 @@ RTPlan rt_plan(const RTCost& cost, int X, int Y, int R, int nsteps, int k_req, i
         }
         if (tile_y > 0) break;
       }
+      if (k_only) break;
     }
   }
   return best;
@@ -127,11 +132,15 @@ bool rt_heat_shape(const Geo& G, int ncomp, const PdeBCRules* rules) {
   if (ncomp != 1 || G.ndims != 2 || G.n[2] != 1 || G.g < G.order / 2 || G.ext[0] < 8 || G.ext[1] < 8 ||
       G.n[0] * G.n[1] >= (1LL << 30))
     return false;
-  // every ghost next to the box is filled by some group (a ghost no group fills keeps its input value)
-  for (int K = 0; rules && K < 27; ++K)
+  return !rules || rt_fills_all_faces(*rules);
+}
+
+// Every ghost next to the box is filled by some group (2D, component 0).
+bool rt_fills_all_faces(const PdeBCRules& rules) {
+  for (int K = 0; K < 27; ++K)
     for (int a = 0; a < 2; ++a) {
       const int k[3] = {K / 9, (K / 3) % 3, K % 3};
-      if (k[2] == 1 && k[a] != 1 && rules->ghost_group[K][a][0] < 0) return false;
+      if (k[2] == 1 && k[a] != 1 && rules.ghost_group[K][a][0] < 0) return false;
     }
   return true;
 }
@@ -154,7 +163,8 @@ RTPlan rt_heat_plan(const Geo& G, int nsteps, int k_req, int tile_x, int tile_y)
   cost.relaunch = 4200.0;
   cost.cell = 130.0;
   cost.shapes = R == 1 ? 15 : 7;
-  return rt_plan(cost, (int)G.ext[0], (int)G.ext[1], R, nsteps, k_req, tile_x, tile_y, sm_count());
+  for (int i = 0; i < 4; ++i) cost.max_warps[i] = rt_heat_warps(i & 1 ? 4 : 2, i & 2 ? 8 : 4);
+  return rt_plan(cost, (int)G.ext[0], (int)G.ext[1], 0, (int)G.ext[0], R, nsteps, k_req, false, tile_x, tile_y, sm_count());
 }
 
 int rt_heat_run(const RTPlan& L, const float* u_in, float* u_out, float* work, const Geo& G,
@@ -191,6 +201,63 @@ int rt_heat_run(const RTPlan& L, const float* u_in, float* u_out, float* work, c
     PDE_CUDA_CHECK(cudaMemcpyAsync(u_out, src, bytes, cudaMemcpyDeviceToDevice, st));
   }
   return PDE_OK;
+}
+
+namespace {
+
+template <int C, int RPT>
+int jacobi_launch(const RTPlan& L, const RJParams& P, const PdeBCRules& rules, cudaStream_t st) {
+  const size_t smem = rt_rows_floats<1, C>(L.threads / 32) * sizeof(float);
+  return launch_pdl(jacobi2d_rt_kernel<C, RPT>, L.tiles, L.threads, smem, st, P, rules);
+}
+
+}  // namespace
+
+RTPlan rt_jacobi_plan(const JacobiRun& J, int nsweeps, int k_req, bool k_only, int tile_x, int tile_y) {
+  RTPlan no;
+  no.ok = false;
+  const int lo = J.held_lo > J.g ? J.held_lo : J.g, hi = J.held_hi < J.X - J.g ? J.held_hi : J.X - J.g;
+  const int o0 = J.own_lo > J.g ? J.own_lo : J.g, o1 = J.own_hi < J.X - J.g ? J.own_hi : J.X - J.g;
+  if (hi - lo < 8 || o1 - o0 < 1 || J.Y - 2 * J.g < 8) return no;
+  RTCost cost = {};
+  cost.ops[0] = 10.0; cost.ops[1] = 8.0; cost.ops[2] = 9.0; cost.ops[3] = 7.0;
+  cost.latency = 220.0;
+  cost.chain = 8.0;
+  cost.barrier = 6.0;
+  cost.relaunch = 4200.0;
+  cost.cell = 180.0;
+  cost.shapes = 15;
+  for (int i = 0; i < 4; ++i) cost.max_warps[i] = RT_WARPS;
+  RTPlan L = rt_plan(cost, hi - lo, J.Y - 2 * J.g, o0 - lo, o1 - lo, 1, nsweeps, k_req, k_only, tile_x, tile_y, sm_count());
+  L.W.xlo = lo == J.g;
+  L.W.xhi = hi == J.X - J.g;
+  return L;
+}
+
+int rt_jacobi_pass(const RTPlan& L, const JacobiRun& J, const float* pin, float* pout, const float* rhs, float* resid,
+                   int k, bool last, const PdeBCRules& rules, cudaStream_t st) {
+  RJParams P;
+  memset(&P, 0, sizeof(P));
+  P.W = L.W;
+  P.X = J.X;
+  P.Y = J.Y;
+  P.g = J.g;
+  P.x0 = J.held_lo > J.g ? J.held_lo : J.g;
+  P.own_lo = J.own_lo;
+  P.own_hi = J.own_hi;
+  P.k = k;
+  P.h2 = J.h2;
+  P.negzero = -0.0f;
+  P.in = pin;
+  P.out = pout;
+  P.rhs = rhs;
+  P.resid = last ? resid : nullptr;
+  switch (L.shape) {
+    case 0: return jacobi_launch<2, 4>(L, P, rules, st);
+    case 1: return jacobi_launch<4, 4>(L, P, rules, st);
+    case 2: return jacobi_launch<2, 8>(L, P, rules, st);
+    default: return jacobi_launch<4, 8>(L, P, rules, st);
+  }
 }
 
 }  // namespace pde

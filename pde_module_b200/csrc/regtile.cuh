@@ -47,9 +47,9 @@ struct RTView {
     warp = (int)threadIdx.x >> 5;
     nw = G.NR / RPT;
     const int tx = tile / G.tiles_y, ty = tile - tx * G.tiles_y;
-    bx0 = tx * G.TBX;
+    bx0 = G.X0 + tx * G.TBX;
     by0 = ty * G.TBY;
-    bx1 = min(bx0 + G.TBX, G.BX);
+    bx1 = min(bx0 + G.TBX, G.X1);
     by1 = min(by0 + G.TBY, G.BY);
     const int rx0 = max(min(bx0 - G.H, G.BX - G.NR), 0), ry0 = max(min(by0 - G.H, G.BY - G.NC), 0);
     r0 = rx0 + warp * RPT;
@@ -59,8 +59,8 @@ struct RTView {
     on = lane <= lh;
     ylo = ry0 == 0;
     yhi = ry0 + G.NC == G.BY;
-    wlo = rx0 == 0 && warp == 0;
-    whi = rx0 + G.NR == G.BX && warp == nw - 1;
+    wlo = G.xlo && rx0 == 0 && warp == 0;
+    whi = G.xhi && rx0 + G.NR == G.BX && warp == nw - 1;
     xe = wlo || whi;
     llo = ylo && lane == 0;
     lhi = yhi && lane == lh;
@@ -294,6 +294,27 @@ __device__ __forceinline__ void rt_store(float2 (&u)[RPT / 2][C], float* p, int 
     if ((tile >> q) & 1u) p[(size_t)(q / C) * pitch + q % C] = rt_at<C, RPT>(u, q / C, q % C);
 }
 
+// The tile, and the ghosts next to it as the last step's fill left them.
+template <int C, int RPT>
+__device__ __forceinline__ void rt_store_all(float2 (&u)[RPT / 2][C], const RTGhosts<C, RPT>& gh,
+                                             const RTView<C, RPT>& V, float* o, int pitch) {
+  constexpr int HP = RPT / 2;
+  const unsigned tile = V.tile_mask();
+  rt_store<C, RPT>(u, o, pitch, tile);
+  if (V.llo || V.lhi) {
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+      if ((tile >> (r * C + (V.llo ? 0 : C - 1))) & 1u)
+        o[(size_t)r * pitch + (V.llo ? -1 : C)] = r < HP ? gh.col[r < HP ? r : 0].x : gh.col[r < HP ? 0 : r - HP].y;
+  }
+  if (V.xe) {
+    float* q = V.wlo ? o - pitch : o + (size_t)RPT * pitch;
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+      if ((tile >> ((V.wlo ? 0 : RPT - 1) * C + j)) & 1u) q[j] = gh.row[j];
+  }
+}
+
 // ---- heat -----------------------------------------------------------------------
 struct RHParams {
   RTGeom W;
@@ -309,8 +330,8 @@ struct RHParams {
 };
 
 // The array's cells outside the box that the fill never writes (corners, and all
-// but the innermost ghost layer) keep the input's values.
-__device__ __forceinline__ void rt_copy_outer(const float* in, float* out, int X, int Y, int g) {
+// but the innermost ghost layer) keep the input's values; rows [lo, hi).
+__device__ __forceinline__ void rt_copy_outer(const float* in, float* out, int X, int Y, int g, int lo, int hi) {
   const int band = g * Y, side = (X - 2 * g) * g, total = 2 * band + 2 * side;
   for (int i = blockIdx.x * (int)blockDim.x + (int)threadIdx.x; i < total; i += (int)(gridDim.x * blockDim.x)) {
     int x, y;
@@ -325,7 +346,7 @@ __device__ __forceinline__ void rt_copy_outer(const float* in, float* out, int X
       y = b % g + (i - 2 * band < side ? 0 : Y - g);
       if (y == g - 1 || y == Y - g) continue;
     }
-    out[(size_t)x * Y + y] = in[(size_t)x * Y + y];
+    if (x >= lo && x < hi) out[(size_t)x * Y + y] = in[(size_t)x * Y + y];
   }
 }
 
@@ -514,7 +535,7 @@ struct RTHeat {
 // exchanged halos through L2 words instead of relaunching cost 2.0 us per exchange
 // against 2.6 us per dependent launch, and nothing at the depths in use: not kept.
 template <int R, int C, int RPT>
-__global__ void __launch_bounds__(rt_max_warps(C, RPT) * 32) heat2d_rt_kernel(const RHParams P, const PdeBCRules Rl) {
+__global__ void __launch_bounds__(rt_heat_warps(C, RPT) * 32) heat2d_rt_kernel(const RHParams P, const PdeBCRules Rl) {
   constexpr int HP = RPT / 2;
   pdl_launch_dependents();  // the next pass may be scheduled; it waits for this one
   extern __shared__ __align__(16) float rows[];
@@ -562,23 +583,145 @@ __global__ void __launch_bounds__(rt_max_warps(C, RPT) * 32) heat2d_rt_kernel(co
     else op.template step<3>(u, V, own + par, E, deep, reach, gh);
     par = flip - par;
   }
-  // the tile, and the ghosts next to it as the last step's fill left them
-  const unsigned tile = V.tile_mask();
-  float* o = P.out + first;
-  rt_store<C, RPT>(u, o, P.Y, tile);
-  if (V.llo || V.lhi) {
+  rt_store_all<C, RPT>(u, gh, V, P.out + first, P.Y);
+  rt_copy_outer(P.in, P.out, P.X, P.Y, P.g, 0, P.X);
+}
+
+// ---- Jacobi sweeps ------------------------------------------------------------------
+struct RJParams {
+  RTGeom W;
+  int X, Y, g;
+  int x0;             // global row of box row 0
+  int own_lo, own_hi; // rows this launch writes (global)
+  int k;
+  float h2, negzero;
+  const float* in;    // arrays addressed by global row
+  float* out;
+  const float* rhs;
+  float* resid;       // if set: the sum of squared updates of the last sweep's tile cells
+};
+
+// k sweeps  p <- 0.25 * ((((pW + pE) + pS) + pN) - h^2 rhs)  of a pass on BC_p(p);
+// h^2 rhs stays in registers.  Bound by issue (arithmetic, shuffles and row exchange
+// share the slots).  50 sweeps on one B200, against cell lists over shared memory
+// (five words of it read and one written per cell and sweep): 1024^2 139 -> 60 us
+// (one 128 x 128 window per SM, 4 x 8 cells a thread), 400^2 31 us, 100^2 24 us.
+template <int C, int RPT>
+__global__ void __launch_bounds__(RT_WARPS * 32) jacobi2d_rt_kernel(const RJParams P, const PdeBCRules Rl) {
+  constexpr int HP = RPT / 2;
+  pdl_launch_dependents();  // the next pass may be scheduled; it waits for this one
+  extern __shared__ __align__(16) float rows[];
+  __shared__ RTBc T;
+  const RTView<C, RPT> V(P.W, blockIdx.x);
+  for (int i = (int)threadIdx.x; i < 21; i += (int)blockDim.x) rt_bc_entry(T, Rl, Rl.dx32, i);
+  __syncthreads();
+  RTGhosts<C, RPT> gh;
+  RTEdge E;
+  if (RPT * C < 32) E.load(T, V);
+  float* const own = rt_own_row<1, C>(rows, V.warp, V.lane);
+  const int flip = (int)rt_buf_floats<1, C>(V.nw);
+  const int ye = (V.ylo ? 1 : 0) | (V.yhi ? 2 : 0);
+  const float2 nz = rt_pair(P.negzero), q4 = rt_pair(0.25f), h2 = rt_pair(P.h2);
+  const size_t first = (size_t)(P.x0 + V.r0) * P.Y + P.g + V.c0;
+  pdl_wait();  // the previous pass's pressure (this pass's input) is complete
+  float2 u[HP][C], hr[HP][C];
+  rt_load<C, RPT>(u, P.in + first, P.Y, V.on);
+  rt_load<C, RPT>(hr, P.rhs + first, P.Y, V.on);
 #pragma unroll
-    for (int r = 0; r < RPT; ++r)
-      if ((tile >> (r * C + (V.llo ? 0 : C - 1))) & 1u)
-        o[(size_t)r * P.Y + (V.llo ? -1 : C)] = r < HP ? gh.col[r < HP ? r : 0].x : gh.col[r < HP ? 0 : r - HP].y;
-  }
-  if (V.xe) {
-    float* q = V.wlo ? o - P.Y : o + (size_t)RPT * P.Y;
+  for (int i = 0; i < HP; ++i)
 #pragma unroll
-    for (int j = 0; j < C; ++j)
-      if ((tile >> ((V.wlo ? 0 : RPT - 1) * C + j)) & 1u) q[j] = gh.row[j];
+    for (int j = 0; j < C; ++j) {
+      const float2 t = __ffma2_rn(h2, hr[i][j], nz);
+      hr[i][j] = make_float2(-t.x, -t.y);  // a - b as a + (-b)
+    }
+  float sq = 0.0f;
+  auto sweep = [&](auto Y, auto N, float* buf, int reach) {
+    constexpr int YE = decltype(Y)::value;
+    constexpr bool norm = decltype(N)::value;  // the step's last sweep: its squared update
+    const bool live = V.dist <= reach + 1;
+    if (live) {
+      if (RPT * C >= 32 && (YE != 0 || V.xe)) E.load(T, V);  // large strips: not kept in registers
+      rt_bc_fill<YE, C, RPT>(u, V, E, gh);
+      rt_publish<1, C, RPT>(buf, u);
+    }
+    float2 le[HP], ri[HP];
+#pragma unroll
+    for (int i = 0; i < HP; ++i) {
+      le[i] = rt_shfl_up(u[i][C - 1]);
+      ri[i] = rt_shfl_down(u[i][0]);
+      if constexpr ((YE & 1) != 0) le[i] = rt_sel(V.llo, gh.col[i], le[i]);
+      if constexpr ((YE & 2) != 0) ri[i] = rt_sel(V.lhi, gh.col[i], ri[i]);
+    }
+    __syncthreads();
+    if (V.dist > reach) return;
+    float up[1][C], dn[1][C];
+    rt_neighbours<1, C>(buf, up, dn);
+    if (V.xe) {
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        up[0][j] = V.wlo ? gh.row[j] : up[0][j];
+        dn[0][j] = V.whi ? gh.row[j] : dn[0][j];
+      }
+    }
+    float2 above[C];  // the old pair of row i - 1
+#pragma unroll
+    for (int j = 0; j < C; ++j) above[j] = make_float2(up[0][j], u[HP - 1][j].x);
+    float2 below_last[C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) below_last[j] = make_float2(u[0][j].y, dn[0][j]);
+    [[maybe_unused]] const unsigned tile = norm ? V.tile_mask() : 0u;
+#pragma unroll
+    for (int i = 0; i < HP; ++i) {
+      float2 nu[C];
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        const float2 dnv = i == HP - 1 ? below_last[j] : u[i + 1 < HP ? i + 1 : i][j];
+        float2 a = __fadd2_rn(above[j], dnv);
+        a = __fadd2_rn(a, j > 0 ? u[i][j > 0 ? j - 1 : 0] : le[i]);
+        a = __fadd2_rn(a, j < C - 1 ? u[i][j < C - 1 ? j + 1 : 0] : ri[i]);
+        nu[j] = __ffma2_rn(q4, __fadd2_rn(a, hr[i][j]), nz);
+      }
+      if constexpr (norm) {
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+          const float dx = nu[j].x - u[i][j].x, dy = nu[j].y - u[i][j].y;
+          if ((tile >> (i * C + j)) & 1u) sq = fmaf(dx, dx, sq);
+          if ((tile >> ((i + HP) * C + j)) & 1u) sq = fmaf(dy, dy, sq);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        above[j] = u[i][j];
+        u[i][j] = nu[j];
+      }
+    }
+  };
+  int par = 0;
+  auto run = [&](auto Y) {
+    for (int reach = P.k - 1; reach >= 0; --reach) {
+      if (reach == 0 && P.resid) sweep(Y, std::true_type{}, own + par, reach);
+      else sweep(Y, std::false_type{}, own + par, reach);
+      par = flip - par;
+    }
+  };
+  if (ye == 0) run(std::integral_constant<int, 0>{});
+  else if (ye == 1) run(std::integral_constant<int, 1>{});
+  else if (ye == 2) run(std::integral_constant<int, 2>{});
+  else run(std::integral_constant<int, 3>{});
+  rt_store_all<C, RPT>(u, gh, V, P.out + first, P.Y);
+  rt_copy_outer(P.in, P.out, P.X, P.Y, P.g, P.own_lo, P.own_hi);
+  if (P.resid) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    __shared__ float wsum[32];
+    if (V.lane == 0) wsum[V.warp] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float b = 0.0f;
+      for (int w = 0; w < V.nw; ++w) b += wsum[w];
+      atomicAdd(P.resid, b);
+    }
   }
-  rt_copy_outer(P.in, P.out, P.X, P.Y, P.g);
 }
 
 }  // namespace pde

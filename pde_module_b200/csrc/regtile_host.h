@@ -5,15 +5,18 @@
 namespace pde {
 
 struct RTGeom {
-  int BX, BY;          // the box the tiles cover
+  int BX, BY;          // the box the windows lie in
+  int X0, X1;          // rows the tiles cover (a slab: its own rows; else 0, BX)
+  bool xlo, xhi;       // the box's first (last) row is a boundary node row (a slab: not at a cut side)
   int TBX, TBY;        // tile
   int tiles_y;
   int H;               // halo (cells)
   int NR, NC;          // window rows (a multiple of RPT) and columns (a multiple of C)
 };
 
-// Warps of a block: 168 registers a thread for 32 cells, 128 for 8 and 16.
-constexpr int rt_max_warps(int C, int RPT) { return C * RPT >= 32 ? 12 : 16; }
+// Most warps of a block: 128 registers a thread; the heat step with 32 cells a thread takes 168.
+constexpr int RT_WARPS = 16;
+constexpr int rt_heat_warps(int C, int RPT) { return C * RPT >= 32 ? 12 : RT_WARPS; }
 
 struct RTCost {
   double ops[4];       // issue cost of a cell and step in lane operations, by shape
@@ -22,6 +25,7 @@ struct RTCost {
   double barrier;      // cycles of a barrier per warp
   double relaunch;     // cycles of a pass besides its steps: the dependent launch ...
   double cell;         // ... and per cell of a thread, its load and store
+  int max_warps[4];    // of a block, by shape
   int shapes;          // bit per (C, RPT) pair: (2,4), (4,4), (2,8), (4,8)
 };
 
@@ -32,12 +36,27 @@ struct RTPlan {
   RTGeom W;
 };
 
-RTPlan rt_plan(const RTCost& cost, int X, int Y, int R, int nsteps, int k_req, int tile_x, int tile_y, int sms);
+// Box of BX x BY cells, tiles over rows [X0, X1).  k_req: deepest pass allowed (0:
+// any); k_only: exactly that depth.
+RTPlan rt_plan(const RTCost& cost, int BX, int BY, int X0, int X1, int R, int nsteps, int k_req, bool k_only,
+               int tile_x, int tile_y, int sms);
 
 bool rt_heat_shape(const Geo& G, int ncomp, const PdeBCRules* rules);
 RTPlan rt_heat_plan(const Geo& G, int nsteps, int k_req, int tile_x, int tile_y);
 int rt_heat_run(const RTPlan& L, const float* u_in, float* u_out, float* work, const Geo& G, const Weights& W,
                 const PdeBCRules& rules, float alpha, float dt, int nsteps, double t0, double tstep, int n0,
                 cudaStream_t st);
+
+// Jacobi sweeps of the cavity's pressure on rows [own_lo, own_hi) of a domain of
+// X x Y cells, arrays holding rows [held_lo, held_hi) (all four in global rows).
+struct JacobiRun {
+  int X, Y, g, own_lo, own_hi, held_lo, held_hi;
+  float h2;
+};
+bool rt_fills_all_faces(const PdeBCRules& rules);
+RTPlan rt_jacobi_plan(const JacobiRun& J, int nsweeps, int k_req, bool k_only, int tile_x, int tile_y);
+// One pass of k sweeps; `last`: add the squared updates of the last sweep to *resid.
+int rt_jacobi_pass(const RTPlan& L, const JacobiRun& J, const float* pin, float* pout, const float* rhs, float* resid,
+                   int k, bool last, const PdeBCRules& rules, cudaStream_t st);
 
 }  // namespace pde

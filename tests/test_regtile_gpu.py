@@ -51,3 +51,23 @@ def test_heat_rollout_unfilled_ghosts_keep_the_shared_memory_path():
         bc.set_BC(name, val, typ, comps)
     got = P.HeatRollout(bc, dx, 0.9, 0.15 * dx * dx)(ud, 13).cpu().numpy()
     assert np.array_equal(got, fdm.heat_rollout(u0, fdm.standard_groups(shape, g, spec), dx, g, 0.9, 0.15 * dx * dx, 13))
+
+
+@pytest.mark.parametrize("n,iters,k", [(8, 5, 0), (17, 9, 3), (62, 50, 0), (64, 7, 7), (129, 50, 0), (300, 33, 8)])
+def test_cavity_window_edges(n, iters, k):
+    """Jacobi windows and the velocity kernels' tiles at one window, one lane or strip
+    more, several tiles; passes of uneven depth; the residual of the last sweep."""
+    s = P.FractionalStepLDC(n=n, Re=100.0, jacobi_iters=iters, jacobi_per_pass=k, dt=1e-3 / n)
+    rng = np.random.default_rng(n)
+    s.u.copy_(torch.from_numpy((0.1 * rng.standard_normal(tuple(s.u.shape))).astype(np.float32)))
+    s.p.copy_(torch.from_numpy((0.1 * rng.standard_normal(tuple(s.p.shape))).astype(np.float32)))
+    u, p = s.u.cpu().numpy(), s.p.cpu().numpy()
+    s.step(2, residuals=True)
+    G = fdm.exterior_groups(u.shape, 1)
+    ug = [dict(ids=G["ALL"], type=1, value=0.0, comps=(0, 1)), dict(ids=G["+Y"], type=1, value=1.0, comps=(0,))]
+    pg = [dict(ids=G["ALL"], type=2, value=0.0, comps=(0,))]
+    for _ in range(2):
+        u, p = fdm.ldc_step(u, p, ug, pg, s.dx, 1, s.nu, s.dt, iters)
+    assert np.array_equal(s.u.cpu().numpy(), u)
+    assert np.array_equal(s.p.cpu().numpy(), p)
+    assert torch.isfinite(s.residuals[:2]).all() and (s.residuals[:2] > 0).all()
