@@ -478,18 +478,19 @@ typedef struct PdeBatchPlan {
   int32_t    total_tiles;
   int32_t    ghost_cells;
   int32_t    order;           /* heat: 2 or 4; wave: 2                              */
-  int32_t    tile_x, tile_y;  /* output tile (cells, ghosts included)               */
+  int32_t    tile_x, tile_y;  /* largest tile of a grid (cells)                     */
   int32_t    steps_per_pass;  /* time-block depth k                                 */
   int32_t    blocks;          /* persistent grid size                               */
   int32_t    smem_bytes;
   PdeBCRules rules;           /* heat: the boundary groups every grid shares        */
+  int32_t    register_tiles;  /* windows in registers (else in shared memory)       */
 } PdeBatchPlan;
 
 /* Device bytes `work` must hold for these grids and tile (0 = default). */
 int pde_batch_work_bytes(const PdeBatchGrid* grids, int32_t ngrids, int32_t tile_x, int32_t tile_y,
                          uint64_t* bytes);
-/* Validate the grids, choose the launch (tile 0 = 32 x 64, steps_per_pass 0 =
- * 8) and upload the descriptor table into `work` on `stream` (from pageable
+/* Validate the grids, choose the launch (tile 0 and steps_per_pass 0: chosen by the
+ * library) and upload the descriptor table into `work` on `stream` (from pageable
  * host memory: call it outside stream capture).  `rules` (heat only; compiled
  * by pde_bc_compile for any grid of the batch, ncomp 1, constant values) is
  * copied into the plan; each grid's own dx is used for its Neumann ghosts.

@@ -92,7 +92,7 @@ class PdeBatchPlan(C.Structure):
     _fields_ = [("table", C.c_void_p), ("kind", C.c_int32), ("ngrids", C.c_int32), ("total_tiles", C.c_int32),
                 ("ghost_cells", C.c_int32), ("order", C.c_int32), ("tile_x", C.c_int32), ("tile_y", C.c_int32),
                 ("steps_per_pass", C.c_int32), ("blocks", C.c_int32), ("smem_bytes", C.c_int32),
-                ("rules", PdeBCRules)]
+                ("rules", PdeBCRules), ("register_tiles", C.c_int32)]
 
 
 class PdeSlab(C.Structure):

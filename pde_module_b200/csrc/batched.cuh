@@ -24,6 +24,7 @@
 #pragma once
 #include "common.cuh"
 #include "fused.cuh"
+#include "regtile_host.h"
 #include "tma.cuh"
 
 namespace pde {
@@ -41,6 +42,7 @@ struct BatchGridDev {
   int ntiles;
   float coef, dt, dx32;  // heat: alpha, dt, dx; wave: K
   float w[5];         // Laplacian weights of this grid's dx
+  RTGeom W;           // register tiles: windows and tiles over the grid's box
 };
 
 struct BatchParams {

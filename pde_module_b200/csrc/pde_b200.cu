@@ -14,6 +14,7 @@
 #include "wave.cuh"
 #include "batched.cuh"
 #include "heat_adj.cuh"
+#include "batched_rt.cuh"
 #include "regtile_host.h"
 
 using namespace pde;
@@ -1531,6 +1532,7 @@ int pde_ldc_slab_step(int32_t phase, float* u, float* u_star, const float* p_in,
 namespace {
 
 constexpr int BATCH_TILE_X = 32, BATCH_TILE_Y = 64, BATCH_K = 8;
+constexpr int BRT_K = 10;  // steps of a time block on register tiles
 constexpr size_t BATCH_QUEUE_OFF_ALIGN = 256;
 
 size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1608,7 +1610,18 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
   const size_t smem = (size_t)nbuf * (tx + 2 * H) * (ty + 2 * H) * sizeof(float);
   if (smem > 227 * 1024) return PDE_ERR_TOO_LARGE;
   BatchGridDev* host = new BatchGridDev[ngrids];
+  // Register tiles where every grid of the batch takes them: order 2, every face
+  // filled (heat), boxes of two strips and two lanes at least, a given tile that fits.
+  const int box_pad = kind == PDE_BATCH_HEAT ? ghost_cells : ghost_cells + 1;
+  const int kr = steps_per_pass > 0 ? steps_per_pass : BRT_K;
+  bool rt = order == 2 && g_dispatch != PDE_DISPATCH_GENERIC && (kind == PDE_BATCH_WAVE || rt_fills_all_faces(*rules));
+  for (int i = 0; i < ngrids && rt; ++i) {
+    const int64_t BX = grids[i].shape[0] - 2 * box_pad, BY = grids[i].shape[1] - 2 * box_pad;
+    rt = BX >= 8 && BY >= 8 && BX * BY < (1LL << 30) &&
+         rt_grid_tiles((int)BX, (int)BY, kr, BRT_C, BRT_RPT, BRT_ROWS, BRT_COLS, tile_x, tile_y, &host[i].W);
+  }
   int64_t base = 0;
+  int most_x = 0, most_y = 0;
   for (int i = 0; i < ngrids; ++i) {
     const PdeBatchGrid& B = grids[i];
     const int64_t X = B.shape[0], Y = B.shape[1];
@@ -1620,6 +1633,7 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
       return X > 2 * ghost_cells + 1 && Y > 2 * ghost_cells + 1 ? PDE_ERR_ARG : PDE_ERR_SHAPE;
     }
     BatchGridDev& D = host[i];
+    const RTGeom win = D.W;
     memset(&D, 0, sizeof(D));
     const size_t cells = (size_t)X * Y;
     D.a0 = B.field;
@@ -1630,6 +1644,13 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
     D.Y = (int)Y;
     D.tiles_y = (int)((Y + ty - 1) / ty);
     D.ntiles = (int)(((X + tx - 1) / tx) * D.tiles_y);
+    if (rt) {
+      D.W = win;
+      D.tiles_y = win.tiles_y;
+      D.ntiles = (win.BX + win.TBX - 1) / win.TBX * win.tiles_y;
+      most_x = win.TBX > most_x ? win.TBX : most_x;
+      most_y = win.TBY > most_y ? win.TBY : most_y;
+    }
     D.tile_base = (int)base;
     base += D.ntiles;
     D.coef = B.coef;
@@ -1642,8 +1663,10 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
   const cudaError_t ce = cudaMemcpyAsync(work, host, (size_t)ngrids * sizeof(BatchGridDev), cudaMemcpyHostToDevice, st);
   delete[] host;
   if (ce != cudaSuccess) return PDE_ERR_CUDA;
-  int occ = 0, rc;
-  if (kind == PDE_BATCH_HEAT)
+  int occ = 0, rc = PDE_OK;
+  if (rt)
+    occ = 2;
+  else if (kind == PDE_BATCH_HEAT)
     rc = order == 2 ? batch_occupancy<BATCH_HEAT, 1>((int)smem, &occ) : batch_occupancy<BATCH_HEAT, 2>((int)smem, &occ);
   else
     rc = batch_occupancy<BATCH_WAVE, 1>((int)smem, &occ);
@@ -1652,12 +1675,13 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
   plan->table = work;
   plan->kind = kind;
   plan->ngrids = ngrids;
-  plan->total_tiles = (int32_t)tiles;
+  plan->total_tiles = rt ? (int32_t)base : (int32_t)tiles;
   plan->ghost_cells = ghost_cells;
   plan->order = order;
-  plan->tile_x = tx;
-  plan->tile_y = ty;
-  plan->steps_per_pass = k;
+  plan->tile_x = rt ? most_x : tx;
+  plan->tile_y = rt ? most_y : ty;
+  plan->steps_per_pass = rt ? kr : k;
+  plan->register_tiles = rt ? 1 : 0;
   plan->blocks = occ * sm_count();
   plan->smem_bytes = (int32_t)smem;
   if (kind == PDE_BATCH_HEAT) plan->rules = *rules;
@@ -1709,7 +1733,10 @@ int batch_rollout_run(const PdeBatchPlan* plan, int32_t nsteps, double t0, void*
   const int64_t items = (int64_t)ntb * plan->total_tiles;
   const int blocks = (int)(items < plan->blocks ? items : plan->blocks);
   const size_t smem = (size_t)plan->smem_bytes;
-  if (plan->kind == PDE_BATCH_HEAT) {
+  if (plan->register_tiles) {
+    if (plan->kind == PDE_BATCH_HEAT) batched_rt_kernel<BATCH_HEAT><<<blocks, BRT_WARPS * 32, 0, st>>>(P, plan->rules, -0.0f);
+    else batched_rt_kernel<BATCH_WAVE><<<blocks, BRT_WARPS * 32, 0, st>>>(P, plan->rules, -0.0f);
+  } else if (plan->kind == PDE_BATCH_HEAT) {
     if (plan->order == 2) batched_kernel<BATCH_HEAT, 1><<<blocks, 256, smem, st>>>(P, plan->rules);
     else batched_kernel<BATCH_HEAT, 2><<<blocks, 256, smem, st>>>(P, plan->rules);
   } else {

@@ -24,7 +24,28 @@ int axis_window(int n, int hold, int nt, int H, int unit, int cap) {
   return win;
 }
 
+// Fewest tiles along an axis of n whose windows of at most cap hold tile and halo.
+int fewest(int n, int hold, int H, int unit, int cap) {
+  if (n == hold && n <= cap && n % unit == 0) return 1;
+  const int two = (n + 1) / 2 + H;
+  if (n == hold && two <= cap / unit * unit && two <= n / unit * unit) return 2;
+  const int room = cap / unit * unit - 2 * H;
+  return room < 1 ? 0 : (n + room - 1) / room;
+}
+
 }  // namespace
+
+bool rt_grid_tiles(int BX, int BY, int H, int C, int RPT, int cap_x, int cap_y, int tile_x, int tile_y, RTGeom* W) {
+  const int nx = tile_x > 0 ? (BX + tile_x - 1) / tile_x : fewest(BX, BX, H, RPT, cap_x);
+  const int ny = tile_y > 0 ? (BY + tile_y - 1) / tile_y : fewest(BY, BY, H, C, cap_y);
+  if (nx < 1 || ny < 1) return false;
+  const int nr = axis_window(BX, BX, nx, H, RPT, cap_x), nc = axis_window(BY, BY, ny, H, C, cap_y);
+  if (nr < 2 * RPT || nc < 2 * C) return false;
+  const int tbx = (BX + nx - 1) / nx, tby = (BY + ny - 1) / ny;
+  if ((nx > 1 && H > tbx) || (ny > 1 && H > tby)) return false;
+  *W = RTGeom{BX, BY, 0, BX, true, true, tbx, tby, ny, H, nr, nc};
+  return true;
+}
 
 // The shape with the least estimated time per step, over the four strips (C, RPT),
 // the pass depths, and per axis the largest windows or as many tiles as fill the
@@ -61,14 +82,6 @@ RTPlan rt_plan(const RTCost& cost, int BX, int Y, int X0, int X1, int R, int nst
     best.W = RTGeom{BX, Y, X0, X1, true, true, tbx, tby, ny, H, nr, nc};
     best.tiles = (int)tiles;
     best.threads = nr / RPT * 32;
-  };
-  // fewest tiles along an axis of n whose windows of at most cap hold tile and halo
-  auto fewest = [](int n, int hold, int H, int unit, int cap) {
-    if (n == hold && n <= cap && n % unit == 0) return 1;
-    const int two = (n + 1) / 2 + H;
-    if (n == hold && two <= cap / unit * unit && two <= n / unit * unit) return 2;
-    const int room = cap / unit * unit - 2 * H;
-    return room < 1 ? 0 : (n + room - 1) / room;
   };
   static const int depths[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 17, 20, 24, 25};
   for (int ci = 0; ci < 4; ++ci) {

@@ -66,16 +66,8 @@ struct RTView {
     lhi = yhi && lane == lh;
   }
   __device__ bool in_tile(int x, int y) const { return x >= bx0 && x < bx1 && y >= by0 && y < by1; }
-  // bit r * C + j: the cell is in the tile
-  __device__ unsigned tile_mask() const {
-    unsigned m = 0;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r)
-#pragma unroll
-      for (int j = 0; j < C; ++j)
-        if (on && in_tile(r0 + r, c0 + j)) m |= 1u << (r * C + j);
-    return m;
-  }
+  __device__ bool row_in(int r) const { return r0 + r >= bx0 && r0 + r < bx1; }           // the same for the whole warp
+  __device__ bool col_in(int j) const { return on && c0 + j >= by0 && c0 + j < by1; }
 };
 
 // Element (row r, column j) of a strip held as pairs.
@@ -287,11 +279,20 @@ __device__ __forceinline__ void rt_load(float2 (&u)[RPT / 2][C], const float* p,
 #pragma unroll
     for (int j = 0; j < C; ++j) rt_at<C, RPT>(u, r, j) = on ? p[(size_t)r * pitch + j] : 0.0f;
 }
+// The tile's cells; rows are in or out for a whole warp, so a row costs one branch
+// and its columns a predicate each.
 template <int C, int RPT>
-__device__ __forceinline__ void rt_store(float2 (&u)[RPT / 2][C], float* p, int pitch, unsigned tile) {
+__device__ __forceinline__ void rt_store(float2 (&u)[RPT / 2][C], float* p, int pitch, const RTView<C, RPT>& V) {
+  bool in[C];
 #pragma unroll
-  for (int q = 0; q < RPT * C; ++q)
-    if ((tile >> q) & 1u) p[(size_t)(q / C) * pitch + q % C] = rt_at<C, RPT>(u, q / C, q % C);
+  for (int j = 0; j < C; ++j) in[j] = V.col_in(j);
+#pragma unroll
+  for (int r = 0; r < RPT; ++r)
+    if (V.row_in(r)) {
+#pragma unroll
+      for (int j = 0; j < C; ++j)
+        if (in[j]) p[(size_t)r * pitch + j] = rt_at<C, RPT>(u, r, j);
+    }
 }
 
 // The tile, and the ghosts next to it as the last step's fill left them.
@@ -299,19 +300,18 @@ template <int C, int RPT>
 __device__ __forceinline__ void rt_store_all(float2 (&u)[RPT / 2][C], const RTGhosts<C, RPT>& gh,
                                              const RTView<C, RPT>& V, float* o, int pitch) {
   constexpr int HP = RPT / 2;
-  const unsigned tile = V.tile_mask();
-  rt_store<C, RPT>(u, o, pitch, tile);
-  if (V.llo || V.lhi) {
+  rt_store<C, RPT>(u, o, pitch, V);
+  if ((V.llo || V.lhi) && V.col_in(V.llo ? 0 : C - 1)) {
 #pragma unroll
     for (int r = 0; r < RPT; ++r)
-      if ((tile >> (r * C + (V.llo ? 0 : C - 1))) & 1u)
+      if (V.row_in(r))
         o[(size_t)r * pitch + (V.llo ? -1 : C)] = r < HP ? gh.col[r < HP ? r : 0].x : gh.col[r < HP ? 0 : r - HP].y;
   }
-  if (V.xe) {
+  if (V.xe && V.row_in(V.wlo ? 0 : RPT - 1)) {
     float* q = V.wlo ? o - pitch : o + (size_t)RPT * pitch;
 #pragma unroll
     for (int j = 0; j < C; ++j)
-      if ((tile >> ((V.wlo ? 0 : RPT - 1) * C + j)) & 1u) q[j] = gh.row[j];
+      if (V.col_in(j)) q[j] = gh.row[j];
   }
 }
 
@@ -669,7 +669,6 @@ __global__ void __launch_bounds__(RT_WARPS * 32) jacobi2d_rt_kernel(const RJPara
     float2 below_last[C];
 #pragma unroll
     for (int j = 0; j < C; ++j) below_last[j] = make_float2(u[0][j].y, dn[0][j]);
-    [[maybe_unused]] const unsigned tile = norm ? V.tile_mask() : 0u;
 #pragma unroll
     for (int i = 0; i < HP; ++i) {
       float2 nu[C];
@@ -685,8 +684,8 @@ __global__ void __launch_bounds__(RT_WARPS * 32) jacobi2d_rt_kernel(const RJPara
 #pragma unroll
         for (int j = 0; j < C; ++j) {
           const float dx = nu[j].x - u[i][j].x, dy = nu[j].y - u[i][j].y;
-          if ((tile >> (i * C + j)) & 1u) sq = fmaf(dx, dx, sq);
-          if ((tile >> ((i + HP) * C + j)) & 1u) sq = fmaf(dy, dy, sq);
+          if (V.row_in(i) && V.col_in(j)) sq = fmaf(dx, dx, sq);
+          if (V.row_in(i + HP) && V.col_in(j)) sq = fmaf(dy, dy, sq);
         }
       }
 #pragma unroll

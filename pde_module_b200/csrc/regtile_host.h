@@ -36,6 +36,11 @@ struct RTPlan {
   RTGeom W;
 };
 
+// Tiles and windows of a box for windows of at most cap_x x cap_y cells, strips of
+// RPT rows and lanes of C columns; false when a window would not fit in the box or
+// its halo would reach past a neighbouring tile.
+bool rt_grid_tiles(int BX, int BY, int H, int C, int RPT, int cap_x, int cap_y, int tile_x, int tile_y, RTGeom* W);
+
 // Box of BX x BY cells, tiles over rows [X0, X1).  k_req: deepest pass allowed (0:
 // any); k_only: exactly that depth.
 RTPlan rt_plan(const RTCost& cost, int BX, int BY, int X0, int X1, int R, int nsteps, int k_req, bool k_only,

@@ -88,8 +88,8 @@ def tune_heat_depth(rollout, u: torch.Tensor, nsteps: int = 256, depths=(1, 2, 4
     return best
 
 
-BATCH_TILES = ((32, 64), (64, 64), (32, 128), (64, 32), (16, 128), (48, 96))
-BATCH_DEPTHS = (2, 4, 6, 8, 12, 16)
+BATCH_TILES = ((0, 0), (32, 64), (64, 64), (32, 128), (64, 32), (16, 128), (48, 96))
+BATCH_DEPTHS = (2, 4, 6, 8, 10, 12, 16)  # tile (0, 0): chosen per grid by the library
 
 
 def tune_batched(rollout, nsteps: int = 100, tiles=BATCH_TILES, depths=BATCH_DEPTHS, reps: int = 2) -> dict:

@@ -71,3 +71,49 @@ def test_cavity_window_edges(n, iters, k):
     assert np.array_equal(s.u.cpu().numpy(), u)
     assert np.array_equal(s.p.cpu().numpy(), p)
     assert torch.isfinite(s.residuals[:2]).all() and (s.residuals[:2] > 0).all()
+
+
+BOXES = [(16, 8), (64, 128), (65, 129), (63, 127), (72, 200), (130, 33), (97, 260)]
+
+
+@pytest.mark.parametrize("k,nsteps", [(0, 23), (4, 9), (12, 1)])
+@pytest.mark.parametrize("spec", [DIRICHLET, MIXED])
+def test_batched_heat_window_edges(k, nsteps, spec):
+    fields = [np.random.default_rng(7 + i).random((x + 2, y + 2, 1, 1)).astype(np.float32) for i, (x, y) in enumerate(BOXES)]
+    dev = [torch.from_numpy(f).cuda() for f in fields]
+    dx = [1.0 / x for x, _ in BOXES]
+    alpha = [0.5 + 0.1 * i for i in range(len(BOXES))]
+    dt = [float(np.float32(0.2 * h * h / a)) for h, a in zip(dx, alpha)]
+    bc = P.GridBoundary(dev[0], dx[0], 1)
+    for name, typ, val, comps in spec:
+        bc.set_BC(name, val, typ, comps)
+    boxes = BOXES[1:] if k == 12 else BOXES  # 16 rows do not hold a window with a halo of 12
+    first = len(BOXES) - len(boxes)
+    roll = P.BatchedHeatRollout(dev[first:], dx[first:], alpha[first:], dt[first:], boundary=bc, steps_per_pass=k)
+    assert roll.plan.register_tiles == 1
+    roll(nsteps)
+    assert P._lib.device_error() == 0
+    for i in range(first, len(BOXES)):
+        ref = fdm.heat_rollout(fields[i], fdm.standard_groups(fields[i].shape[:3], 1, spec), dx[i], 1, alpha[i], dt[i], nsteps)
+        assert np.array_equal(dev[i].cpu().numpy(), ref), BOXES[i]
+
+
+@pytest.mark.parametrize("k,nsteps", [(0, 23), (4, 9), (8, 2)])
+def test_batched_wave_window_edges(k, nsteps):
+    boxes = [(x + 2, y + 2) for x, y in BOXES]  # the wave's box leaves out the node ring
+    u = []
+    for i, (x, y) in enumerate(boxes):
+        f = np.zeros((x + 2, y + 2, 1, 1), dtype=np.float32)
+        f[2:-2, 2:-2, 0, 0] = np.random.default_rng(70 + i).standard_normal((x - 2, y - 2))
+        u.append(f)
+    K = [float(np.float32(0.2 / (x * x))) for x, _ in boxes]
+    dx = [1.0 / x for x, _ in boxes]
+    now, prev = [torch.from_numpy(f).cuda() for f in u], [torch.from_numpy(f).cuda() for f in u]
+    roll = P.BatchedWaveRollout(now, prev, dx, K, steps_per_pass=k)
+    assert roll.plan.register_tiles == 1
+    roll(nsteps)
+    assert P._lib.device_error() == 0
+    for i in range(len(boxes)):
+        st = fdm.wave_forward(np.full(u[i].shape, K[i], np.float32), u[i], None, -1, nsteps, dx[i])
+        assert np.array_equal(now[i].cpu().numpy()[:, :, 0, 0], st[-1]), boxes[i]
+        assert np.array_equal(prev[i].cpu().numpy()[:, :, 0, 0], st[-2]), boxes[i]
