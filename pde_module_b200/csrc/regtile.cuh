@@ -565,24 +565,27 @@ __global__ void __launch_bounds__(rt_heat_warps(C, RPT) * 32) heat2d_rt_kernel(c
   int par = 0;
   // Step s only has to update the cells within R (k - 1 - s) of the tile: the
   // strips beyond that rest.  The fill and the rows are needed one R further.
-  for (int reach = R * (P.k - 1); reach >= 0; reach -= R) {
-    if (Rl.has_ramp) {
-      // every read of the table in the previous step came before its barrier
-      if (tid < Rl.ngroups && Rl.group[tid].func == PDE_BC_FUNC_RAMP) {
-        const float t = step_time(P.t0, P.tstep, P.n0 + P.k - 1 - reach / R);
-        SR.group[tid].value = bc_value(PDE_BC_FUNC_RAMP, Rl.group[tid].value, Rl.group[tid].t_max, &t);
+  auto run = [&](auto Y) {
+    for (int reach = R * (P.k - 1); reach >= 0; reach -= R) {
+      if (Rl.has_ramp) {
+        // every read of the table in the previous step came before its barrier
+        if (tid < Rl.ngroups && Rl.group[tid].func == PDE_BC_FUNC_RAMP) {
+          const float t = step_time(P.t0, P.tstep, P.n0 + P.k - 1 - reach / R);
+          SR.group[tid].value = bc_value(PDE_BC_FUNC_RAMP, Rl.group[tid].value, Rl.group[tid].t_max, &t);
+        }
+        __syncthreads();
+        for (int i = tid; i < 21; i += nt) rt_bc_entry(T, SR, Rl.dx32, i);
+        __syncthreads();
+        E.load(T, V);
       }
-      __syncthreads();
-      for (int i = tid; i < 21; i += nt) rt_bc_entry(T, SR, Rl.dx32, i);
-      __syncthreads();
-      E.load(T, V);
+      op.template step<decltype(Y)::value>(u, V, own + par, E, deep, reach, gh);
+      par = flip - par;
     }
-    if (ye == 0) op.template step<0>(u, V, own + par, E, deep, reach, gh);
-    else if (ye == 1) op.template step<1>(u, V, own + par, E, deep, reach, gh);
-    else if (ye == 2) op.template step<2>(u, V, own + par, E, deep, reach, gh);
-    else op.template step<3>(u, V, own + par, E, deep, reach, gh);
-    par = flip - par;
-  }
+  };
+  if (ye == 0) run(std::integral_constant<int, 0>{});
+  else if (ye == 1) run(std::integral_constant<int, 1>{});
+  else if (ye == 2) run(std::integral_constant<int, 2>{});
+  else run(std::integral_constant<int, 3>{});
   rt_store_all<C, RPT>(u, gh, V, P.out + first, P.Y);
   rt_copy_outer(P.in, P.out, P.X, P.Y, P.g, 0, P.X);
 }
