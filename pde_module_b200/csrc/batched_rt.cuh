@@ -38,72 +38,17 @@ __device__ __forceinline__ void brt_load(float2 (&u)[BRT_RPT / 2][BRT_C], const 
   }
 }
 
-// A step's sums, a row pair at a time: calls put(i, j, mid, lap) with lap the
-// reference's Laplacian sum (alpha 1) of pair (i, j).  Products of the outer weight
-// are formed once per cell: the strip's first and last rows before the barrier, as
-// the warps exchange them, the others as the rows go by.  edge_row / edge_col:
-// values beyond the box's ends (fill functions of the caller).
-template <int YE, class Fill, class Put>
+// One step: fill (boundary, if any), row exchange, sums through put.
+template <int YE, bool ZERO, class Fill, class Put>
 __device__ __forceinline__ void brt_step(float2 (&u)[BRT_RPT / 2][BRT_C], const RTView<BRT_C, BRT_RPT>& V, float* buf,
                                          float2 w0, float2 nz, int reach, const RTGhosts<BRT_C, BRT_RPT>& gh,
                                          Fill fill, Put put) {
-  constexpr int C = BRT_C, HP = BRT_RPT / 2;
-  auto M = [&](float2 a, float2 b) { return __ffma2_rn(a, b, nz); };
   const bool live = V.dist <= reach + 1;
   if (live) fill();
-  float2 cur[C], last[C];
-#pragma unroll
-  for (int j = 0; j < C; ++j) {
-    cur[j] = M(w0, u[0][j]);
-    last[j] = M(w0, u[HP - 1][j]);
-  }
-  if (live) {
-    float top[C], bot[C];
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      top[j] = cur[j].x;
-      bot[j] = last[j].y;
-    }
-    rt_put<C>(buf, top);
-    rt_put<C>(buf + 32 * C, bot);
-  }
+  RTRows<BRT_C> e;
+  rt_rows_put<BRT_C, BRT_RPT>(u, buf, w0, nz, live, e);
   __syncthreads();
-  if (V.dist > reach) return;
-  float up[C], dn[C];
-  rt_get<C>(buf - 32 * C, up);
-  rt_get<C>(buf + 2 * 32 * C, dn);
-  if (V.xe) {
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const float q = mul(w0.x, gh.row[j]);
-      up[j] = V.wlo ? q : up[j];
-      dn[j] = V.whi ? q : dn[j];
-    }
-  }
-  float2 above[C], below[C];
-#pragma unroll
-  for (int j = 0; j < C; ++j) {
-    above[j] = make_float2(up[j], last[j].x);
-    below[j] = make_float2(cur[j].y, dn[j]);
-  }
-#pragma unroll
-  for (int i = 0; i < HP; ++i) {
-    float2 next[C];
-#pragma unroll
-    for (int j = 0; j < C; ++j)
-      next[j] = i == HP - 1 ? below[j] : (i == HP - 2 ? last[j] : M(w0, u[i + 1 < HP ? i + 1 : i][j]));
-    float2 le = rt_shfl_up(cur[C - 1]), ri = rt_shfl_down(cur[0]);
-    if constexpr ((YE & 1) != 0) le = rt_sel(V.llo, M(w0, gh.col[i]), le);
-    if constexpr ((YE & 2) != 0) ri = rt_sel(V.lhi, M(w0, gh.col[i]), ri);
-#pragma unroll
-    for (int j = 0; j < C; ++j)
-      put(i, j, above[j], next[j], j > 0 ? cur[j > 0 ? j - 1 : 0] : le, j < C - 1 ? cur[j < C - 1 ? j + 1 : 0] : ri);
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      above[j] = cur[j];
-      cur[j] = next[j];
-    }
-  }
+  if (V.dist <= reach) rt_rows_sum<YE, ZERO, BRT_C, BRT_RPT>(u, V, buf, w0, nz, e, gh, put);
 }
 
 template <int OP>
@@ -190,7 +135,7 @@ __global__ void __launch_bounds__(BRT_WARPS * 32, 2) batched_rt_kernel(const Bat
             __syncthreads();
             continue;
           }
-          brt_step<YE>(
+          brt_step<YE, false>(
               u, V, own + par, w0, nz, reach, gh,
               [&]() {
                 if (YE != 0 || V.xe) {
@@ -232,15 +177,11 @@ __global__ void __launch_bounds__(BRT_WARPS * 32, 2) batched_rt_kernel(const Bat
         brt_load(u, in0 + first, Gd.Y, V, W.H);
         brt_load(um, in1 + first, Gd.Y, V, W.H);
       }
-      RTGhosts<C, RPT> gh;  // zero beyond the ring
-#pragma unroll
-      for (int i = 0; i < HP; ++i) gh.col[i] = rt_pair(0.0f);
-#pragma unroll
-      for (int j = 0; j < C; ++j) gh.row[j] = 0.0f;
+      RTGhosts<C, RPT> gh;  // not read: 0 beyond the ring
       const float2 two = rt_pair(2.0f);
       by_edge([&](auto Y) {
         auto step = [&](float2 (&now)[HP][C], float2 (&old)[HP][C], int reach) {  // the new level over the old one
-          brt_step<decltype(Y)::value>(now, V, own + par, w0, nz, reach, gh, []() {},
+          brt_step<decltype(Y)::value, true>(now, V, own + par, w0, nz, reach, gh, []() {},
                                        [&](int i, int j, float2 a, float2 b, float2 l, float2 r) {
                                          const float2 mid = M(w1, now[i][j]);
                                          float2 acc = __fadd2_rn(a, mid);

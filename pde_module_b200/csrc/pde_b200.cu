@@ -1028,15 +1028,23 @@ bool wave_setup(const PdeGrid* grid, int steps_per_pass, int nsteps, Geo* G, Wav
   return *smem <= 227 * 1024;
 }
 
-// Register cell lists of the wave kernels: the region capacity bounds every
-// block's rectangle, so MAXC (4, 6 or 8) cells per thread cover it; 0 = the
-// general loop (rectangles beyond 8 cells per thread).
-int wave_cells_per_thread(int rc, int threads) {
-  if (rc <= 4 * threads) return 4;
-  if (rc <= 6 * threads) return 6;
-  if (rc <= 8 * threads) return 8;
-  return 0;
+// The register-tile passes of a wave call (wave_rt.cuh); the shared-memory kernels
+// take boxes under 8 cells a side, tiles set too large for a window, and the
+// general dispatch.
+WaveRun wave_run(const WaveParams& P, const float* K, int srcx, int srcy) {
+  WaveRun J{P.X, P.Y, P.g, {P.w[0], P.w[1]}, K, srcx, srcy};
+  return J;
 }
+RTPlan wave_plan(const WaveRun& J, bool fwd, bool adj, int nsteps, int steps_per_pass) {
+  if (g_dispatch == PDE_DISPATCH_GENERIC) {
+    RTPlan no;
+    no.ok = false;
+    return no;
+  }
+  return rt_wave_plan(J, fwd, adj, nsteps, steps_per_pass, g_tile2d[0], g_tile2d[1]);
+}
+// Depth of pass `pass` of `npasses` when `left` steps remain: even shares.
+int pass_depth(int left, int passes_left) { return (left + passes_left - 1) / passes_left; }
 
 }  // namespace
 
@@ -1065,9 +1073,11 @@ int pde_wave_forward(const float* K, const float* u_prev, const float* u_cur, fl
   }
   const int tiles = ((P.X + P.TBX - 1) / P.TBX) * P.tiles_y;
   const int threads = pick_threads_2d(tiles);
-  const int cpt = wave_cells_per_thread(P.RC, threads);
-  auto kern = cpt == 4 ? wave_fwd_tb_kernel<4> : cpt == 6 ? wave_fwd_tb_kernel<6> : cpt == 8 ? wave_fwd_tb_kernel<8> : wave_fwd_tb_kernel<0>;
-  PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const WaveRun J = wave_run(P, K, P.srcx, P.srcy);
+  const RTPlan L = wave_plan(J, true, false, nsteps, steps_per_pass);
+  auto kern = wave_fwd_tb_kernel;
+  if (L.ok) k = L.k;
+  else PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int npasses = (nsteps + k - 1) / k;
   float* w0 = work;
   float* w1 = work + P.cells;
@@ -1077,13 +1087,19 @@ int pde_wave_forward(const float* K, const float* u_prev, const float* u_cur, fl
   const float* b = u_cur;
   int done = 0;
   for (int p = 0; p < npasses; ++p) {
-    P.k = (nsteps - done < k) ? (nsteps - done) : k;
+    P.k = pass_depth(nsteps - done, npasses - p);
     P.n0 = n0 + done;
     P.lst = lstates ? lstates + (size_t)done * P.cells : nullptr;
     float* da = to_out ? out_prev : w0;
     float* db = to_out ? out_cur : w1;
-    kern<<<tiles, threads, smem, st>>>(a, b, K, da, db, P);
-    const int rc = launch_status();
+    int rc;
+    if (L.ok) {
+      const WaveFwd f{P.k, a, b, da, db, P.lst, src_cell >= 0 ? src + P.n0 : nullptr};
+      rc = rt_wave_pass(L, J, &f, nullptr, st);
+    } else {
+      kern<<<tiles, threads, smem, st>>>(a, b, K, da, db, P);
+      rc = launch_status();
+    }
     if (rc) return rc;
     a = da;
     b = db;
@@ -1131,13 +1147,11 @@ int pde_wave_pair(const float* K, const float* u_prev, const float* u_cur, int32
   const size_t bytes = sizeof(float) * (size_t)Pa.cells;
   const int tiles = ((Pa.X + Pa.TBX - 1) / Pa.TBX) * Pa.tiles_y;
   const int threads = pick_threads_2d(tiles);
-  const int cpt = wave_cells_per_thread(Pa.RC, threads);
-  // register lists: the packed kernel (two cells per slot, cpt/2 slots); beyond 8
-  // cells per thread the general loop
-  auto kern = cpt == 4 ? wave_pair2_tb_kernel<2> : cpt == 6 ? wave_pair2_tb_kernel<3> : wave_pair2_tb_kernel<4>;
-  auto kern0 = wave_pair_tb_kernel;
-  if (cpt > 0) PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  else PDE_CUDA_CHECK(cudaFuncSetAttribute(kern0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const WaveRun J = wave_run(Pa, K, Pf.srcx, Pf.srcy);
+  const RTPlan L = wave_plan(J, nsteps_fwd > 0, nsteps_adj > 0, nmax, steps_per_pass);
+  auto kern = wave_pair_tb_kernel;
+  if (L.ok) k = L.k;
+  else PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   float* w[6];
   for (int i = 0; i < 6; ++i) w[i] = work + (size_t)i * Pa.cells;
   // forward part: (u_prev, u_cur) -> (w0, w1) -> (w2, w3) -> (w0, w1) ...; the inputs are never written
@@ -1160,9 +1174,15 @@ int pde_wave_pair(const float* K, const float* u_prev, const float* u_cur, int32
     float* fo_b = w[2 * fslot + 1];
     float* mo_a = to_out ? mu_out : w[4];
     float* mo_b = to_out ? mu_out_next : w[5];
-    if (cpt > 0) kern<<<tiles, threads, smem, st>>>(fa, fb, fo_a, fo_b, ma, mb, mo_a, mo_b, K, Pf, Pa, -0.0f);
-    else kern0<<<tiles, threads, smem, st>>>(fa, fb, fo_a, fo_b, ma, mb, mo_a, mo_b, K, Pf, Pa);
-    const int rc = launch_status();
+    int rc;
+    if (L.ok) {
+      const WaveFwd f{Pf.k, fa, fb, fo_a, fo_b, Pf.lst, src_cell >= 0 ? src + Pf.n0 : nullptr};
+      const WaveAdj a{Pa.k, ma, mb, mo_a, mo_b, Pa.lsts + (ptrdiff_t)Pa.ntop * Pa.cells, grad_K};
+      rc = rt_wave_pass(L, J, Pf.k > 0 ? &f : nullptr, Pa.k > 0 ? &a : nullptr, st);
+    } else {
+      kern<<<tiles, threads, smem, st>>>(fa, fb, fo_a, fo_b, ma, mb, mo_a, mo_b, K, Pf, Pa);
+      rc = launch_status();
+    }
     if (rc) return rc;
     if (Pf.k > 0) {
       fa = fo_a;
@@ -1198,9 +1218,11 @@ int pde_wave_adjoint(const float* K, const float* mu_next, const float* mu_next2
   const size_t bytes = sizeof(float) * (size_t)P.cells;
   const int tiles = ((P.X + P.TBX - 1) / P.TBX) * P.tiles_y;
   const int threads = pick_threads_2d(tiles);
-  const int cpt = wave_cells_per_thread(P.RC, threads);
-  auto kern = cpt == 4 ? wave_adj_tb_kernel<4> : cpt == 6 ? wave_adj_tb_kernel<6> : cpt == 8 ? wave_adj_tb_kernel<8> : wave_adj_tb_kernel<0>;
-  PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const WaveRun J = wave_run(P, K, -1, -1);
+  const RTPlan L = wave_plan(J, false, true, nsteps, steps_per_pass);
+  auto kern = wave_adj_tb_kernel;
+  if (L.ok) k = L.k;
+  else PDE_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int npasses = (nsteps + k - 1) / k;
   float* w0 = work;
   float* w1 = work + P.cells;
@@ -1216,8 +1238,14 @@ int pde_wave_adjoint(const float* K, const float* mu_next, const float* mu_next2
     P.ntop = nsteps - 1 - done;
     float* da = to_out ? mu_out : w0;
     float* db = to_out ? mu_out_next : w1;
-    kern<<<tiles, threads, smem, st>>>(a, b, K, da, db, P);
-    const int rc = launch_status();
+    int rc;
+    if (L.ok) {
+      const WaveAdj q{P.k, a, b, da, db, lstates + (size_t)P.ntop * P.cells, grad_K};
+      rc = rt_wave_pass(L, J, nullptr, &q, st);
+    } else {
+      kern<<<tiles, threads, smem, st>>>(a, b, K, da, db, P);
+      rc = launch_status();
+    }
     if (rc) return rc;
     a = da;
     b = db;

@@ -62,10 +62,19 @@ RTPlan rt_plan(const RTCost& cost, int BX, int Y, int X0, int X1, int R, int nst
   best.cycles = 1e30;
   auto consider = [&](int ci, int C, int RPT, int k, int nx, int ny) {
     const int H = k * R;
-    const int nr = axis_window(X, BX, nx, H, RPT, cost.max_warps[ci] * RPT), nc = axis_window(Y, Y, ny, H, C, 32 * C);
+    const int nr = axis_window(X, BX, nx, H, RPT, cost.max_warps[ci] * RPT);
+    int nc = axis_window(Y, Y, ny, H, C, 32 * C);
     if (nr < 2 * RPT || nc < 2 * C) return;
     const long long tiles = (long long)nx * ny;
-    const int tbx = (X + nx - 1) / nx, tby = (Y + ny - 1) / ny;
+    const int tbx = (X + nx - 1) / nx;
+    int tby = (Y + ny - 1) / ny;
+    if (cost.even && ny > 1 && (tby & 1) && (ny - 1) * (tby + 1) < Y) {
+      const int wide = (tby + 1 + (ny == 2 ? 1 : 2) * H + C - 1) / C * C;
+      if (wide <= 32 * C && wide <= Y) {
+        ++tby;
+        nc = wide > nc ? wide : nc;
+      }
+    }
     const double act = fmin((double)nr, tbx + 1.4 * H + RPT);  // strips rest as the reach shrinks
     const double per_sm = (double)((tiles + sms - 1) / sms);
     const double arith = act * 32.0 * C * cost.ops[ci] / 128.0 * per_sm;
@@ -89,6 +98,7 @@ RTPlan rt_plan(const RTCost& cost, int BX, int Y, int X0, int X1, int R, int nst
     const int C = ci & 1 ? 4 : 2, RPT = ci & 2 ? 8 : 4;
     for (int d : depths) {
       const int k = k_only ? k_req : d;
+      if (cost.even && (k & 1) && k != nsteps && k != k_req && k > 1) continue;
       if (k > nsteps || (k_req > 0 && k > k_req)) break;
       int ny = tile_y > 0 ? (Y + tile_y - 1) / tile_y : fewest(Y, Y, k * R, C, 32 * C);
       if (ny < 1) break;

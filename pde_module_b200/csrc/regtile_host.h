@@ -26,6 +26,7 @@ struct RTCost {
   double relaunch;     // cycles of a pass besides its steps: the dependent launch ...
   double cell;         // ... and per cell of a thread, its load and store
   int max_warps[4];    // of a block, by shape
+  bool even;           // even depths and tile widths (column pairs that stay together)
   int shapes;          // bit per (C, RPT) pair: (2,4), (4,4), (2,8), (4,8)
 };
 
@@ -63,5 +64,28 @@ RTPlan rt_jacobi_plan(const JacobiRun& J, int nsweeps, int k_req, bool k_only, i
 // One pass of k sweeps; `last`: add the squared updates of the last sweep to *resid.
 int rt_jacobi_pass(const RTPlan& L, const JacobiRun& J, const float* pin, float* pout, const float* rhs, float* resid,
                    int k, bool last, const PdeBCRules& rules, cudaStream_t st);
+
+// Wave passes (wave_rt.cuh): forward, adjoint, or both of equal depth in one launch.
+struct WaveRun {
+  int X, Y, g;
+  float w[2];
+  const float* K;
+  int srcx, srcy;  // array coordinates, -1: none
+};
+struct WaveFwd {
+  int k;
+  const float *um, *u0;
+  float *um_out, *u0_out, *lst;
+  const float* src;
+};
+struct WaveAdj {
+  int k;
+  const float *m1, *m2;
+  float *m1_out, *m2_out;
+  const float* lsts;
+  float* gK;
+};
+RTPlan rt_wave_plan(const WaveRun& J, bool fwd, bool adj, int nsteps, int k_req, int tile_x, int tile_y);
+int rt_wave_pass(const RTPlan& L, const WaveRun& J, const WaveFwd* f, const WaveAdj* a, cudaStream_t st);
 
 }  // namespace pde

@@ -82,50 +82,6 @@ struct WaveRect {
   }
 };
 
-// The rectangle cells of this thread: its slots q = threadIdx.x + c * blockDim.x
-// (c < MAXC) walk the rectangle's rows at their full region width RY, the
-// columns outside the rectangle left idle, so a warp's 32 slots are 32
-// consecutive region cells (NB-float stride in shared memory: no bank
-// conflicts) and no warp straddles the gap between two rectangle rows.  The
-// same cells in every step (the rectangle is fixed for the pass), so their
-// indices, the gradient sums of the tile cells among them and the next step's
-// L(u^n) values stay in registers.  Needs NR * RY <= MAXC * blockDim.x.
-// dist: the cell's distance from the tile (the larger of its x and y distances).
-// Step s of a k-step pass only has to update cells with dist <= k - 1 - s: the
-// tile's values after the pass depend on no other cell, so the rest is skipped.
-template <int MAXC>
-struct WaveCells {
-  int ri[MAXC];    // region index; -1 for an idle slot
-  int gi[MAXC];    // array index of a tile cell; 0 (a valid address) for the other cells
-  int dist[MAXC];  // distance from the tile; 1 << 20 for an idle slot
-  unsigned tile;   // bit c: slot c holds a tile cell
-  __device__ bool is_tile(int c) const { return (tile >> c) & 1u; }
-  __device__ WaveCells(const WaveRect& Rt, const WaveRegion& Rg, int Y) {
-    const int nt = (int)blockDim.x;
-    // tile origin: rows relative to the rectangle, columns relative to the region
-    const int tx0 = Rg.bx0 - Rg.rx0 - Rt.cx0, ty0 = Rg.by0 - Rg.ry0;
-    const int n = Rt.NR * Rg.RY;
-    RectWalk wk(Rg.RY, nt);
-    tile = 0;
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      ri[c] = -1;
-      gi[c] = 0;
-      dist[c] = 1 << 20;
-      if ((int)threadIdx.x + c * nt < n && wk.col >= Rt.cy0 && wk.col < Rt.cy0 + Rt.W) {
-        ri[c] = (Rt.cx0 + wk.row) * Rg.RY + wk.col;
-        const int ox = wk.row - tx0, oy = wk.col - ty0;
-        if (ox >= 0 && ox < Rg.OX && oy >= 0 && oy < Rg.OY) {
-          gi[c] = (Rg.bx0 + ox) * Y + Rg.by0 + oy;
-          tile |= 1u << c;
-        }
-        dist[c] = max(max(max(-ox, ox - (Rg.OX - 1)), max(-oy, oy - (Rg.OY - 1))), 0);
-      }
-      wk.next();
-    }
-  }
-};
-
 // Load a region row-major (RX x RY) with fn(region index, array x, array y).
 template <class F>
 __device__ __forceinline__ void for_region(const WaveRegion& Rg, F fn) {
@@ -155,17 +111,6 @@ __device__ __forceinline__ void for_tile(const WaveRegion& Rg, int Y, F fn) {
 //   adjoint  (NB 5): 0, 1 levels of mu (mu^{n+1} in 1 - p), 2, 3 levels of K o mu
 //                    (K o mu^{n+1} in 3 - p), 4 K
 //   paired   (NB 7): 0, 1 u; 2, 3 mu; 4, 5 K o mu; 6 K
-template <int V>
-using IC = std::integral_constant<int, V>;
-
-// st.global under a predicate, without a branch around it
-__device__ __forceinline__ void st_global_if(float* p, float v, bool on) {
-  asm volatile(
-      "{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q st.global.f32 [%0], %1;\n}\n" ::"l"(p), "f"(v),
-      "r"((int)on)
-      : "memory");
-}
-
 // Laplacian (alpha 1) around the interleaved element c: rows rs floats apart,
 // neighbours along y NB floats apart; the reference's term order.
 template <int NB>
@@ -188,41 +133,12 @@ __device__ __forceinline__ int wave_src_index(const WaveParams& P, const WaveReg
 }
 
 // k forward steps: u^{n+1} = 2 u^n - u^{n-1} + K o L(u^n) (+ source), written over u^{n-1}.
-template <bool STORE, int MAXC>
+template <bool STORE>
 __device__ __forceinline__ void wave_fwd_steps(const WaveParams& P, const WaveRegion& Rg, float* sm) {
   constexpr int NB = 3;
   const int RY = Rg.RY, rs = NB * RY;
   const WaveRect Rt(P, Rg);
   const int srci = wave_src_index(P, Rg);
-  if constexpr (MAXC > 0) {
-    const WaveCells<MAXC> C(Rt, Rg, P.Y);
-    float kc[MAXC];  // K of the thread's cells (constant over the pass)
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) kc[c] = C.ri[c] >= 0 ? sm[NB * C.ri[c] + 2] : 0.0f;
-    auto step = [&](auto PAR, int s) {
-      constexpr int p = decltype(PAR)::value;
-      const float sn = (srci >= 0) ? P.src[P.n0 + s] : 0.0f;
-      float* Ls = STORE ? P.lst + (size_t)s * P.cells : nullptr;
-      const int reach = P.k - 1 - s;
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) {
-        if (C.dist[c] > reach) continue;  // past the rectangle: dist is out of reach
-        float* pc = sm + NB * C.ri[c];
-        const float lap = lap5n<NB>(pc + (1 - p), rs, P.w);
-        float v = sub(mul(2.0f, pc[1 - p]), pc[p]);
-        v = add(v, mul(kc[c], lap));
-        if (C.ri[c] == srci) v = add(v, sn);
-        pc[p] = v;
-        if (STORE) st_global_if(Ls + C.gi[c], lap, C.is_tile(c));
-      }
-      __syncthreads();
-    };
-    for (int s = 0; s < P.k; s += 2) {
-      step(IC<0>{}, s);
-      if (s + 1 < P.k) step(IC<1>{}, s + 1);
-    }
-    return;
-  }
   // the tile in rectangle coordinates (for the stored Laplacians)
   const int nt = (int)blockDim.x;
   const int tx0 = Rg.bx0 - Rg.rx0 - Rt.cx0, ty0 = Rg.by0 - Rg.ry0 - Rt.cy0;
@@ -249,7 +165,6 @@ __device__ __forceinline__ void wave_fwd_steps(const WaveParams& P, const WaveRe
   }
 }
 
-template <int MAXC>
 __global__ void __launch_bounds__(1024) wave_fwd_tb_kernel(const float* __restrict__ um_in,
                                                             const float* __restrict__ u0_in,
                                                             const float* __restrict__ Kf, float* __restrict__ um_out,
@@ -266,8 +181,8 @@ __global__ void __launch_bounds__(1024) wave_fwd_tb_kernel(const float* __restri
   });
   cp_async_wait_all();
   __syncthreads();
-  if (P.lst) wave_fwd_steps<true, MAXC>(P, Rg, sm);
-  else wave_fwd_steps<false, MAXC>(P, Rg, sm);
+  if (P.lst) wave_fwd_steps<true>(P, Rg, sm);
+  else wave_fwd_steps<false>(P, Rg, sm);
   const int nw = (P.k & 1) ? 0 : 1;  // level the last step wrote
   for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) {
     um_out[gi] = sm[NB * ri + (1 - nw)];
@@ -275,10 +190,6 @@ __global__ void __launch_bounds__(1024) wave_fwd_tb_kernel(const float* __restri
   });
 }
 
-// MAXC > 0: the cells of a thread in registers (WaveCells), the gradient sums
-// of its tile cells in registers and L(u^n) of the next step loaded while this
-// one computes; MAXC = 0: any rectangle size, gradient tile in shared memory.
-template <int MAXC>
 __global__ void __launch_bounds__(1024) wave_adj_tb_kernel(const float* __restrict__ m1_in,
                                                             const float* __restrict__ m2_in,
                                                             const float* __restrict__ Kf, float* __restrict__ m1_out,
@@ -287,7 +198,7 @@ __global__ void __launch_bounds__(1024) wave_adj_tb_kernel(const float* __restri
   constexpr int NB = 5;
   const WaveRegion Rg(P, P.k);
   const int RY = Rg.RY, rs = NB * RY;
-  const int oga = NB * P.RC;  // dJ/dK of the tile (MAXC = 0)
+  const int oga = NB * P.RC;  // dJ/dK of the tile
   for_region(Rg, [&](int i, int x, int y) {
     const size_t gi = (size_t)x * P.Y + y;
     const bool in = wave_inside(P, x, y);
@@ -296,82 +207,38 @@ __global__ void __launch_bounds__(1024) wave_adj_tb_kernel(const float* __restri
     cp_async4(sm + NB * i + 4, Kf + gi, true);
     sm[NB * i + 2] = 0.0f;
   });
-  if (MAXC == 0) for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) { cp_async4(sm + oga + t, P.gK + gi, true); });
+  for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) { cp_async4(sm + oga + t, P.gK + gi, true); });
   cp_async_wait_all();
   // K o mu^{n+1} of the cells this thread copied (its own copies are complete)
   for_region(Rg, [&](int i, int x, int y) { sm[NB * i + 3] = mul(sm[NB * i + 4], sm[NB * i + 1]); });
   __syncthreads();
   const WaveRect Rt(P, Rg);
-  if constexpr (MAXC > 0) {
-    const WaveCells<MAXC> C(Rt, Rg, P.Y);
-    // lv: L(u^n) of the step at the thread's cells, the next step's issued before
-    // each barrier; the other cells load from index 0 and their gradient sums go
-    // unused (no per-cell branches)
-    float ga[MAXC], lv[MAXC], kc[MAXC];
-    const float* L0 = P.lsts + (size_t)P.ntop * P.cells;
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      ga[c] = C.is_tile(c) ? P.gK[C.gi[c]] : 0.0f;
-      lv[c] = __ldg(L0 + C.gi[c]);
-      kc[c] = C.ri[c] >= 0 ? sm[NB * C.ri[c] + 4] : 0.0f;  // K of the thread's cells
-    }
-    auto step = [&](auto PAR, int s) {
-      constexpr int p = decltype(PAR)::value;
-      const int reach = P.k - 1 - s;
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) {
-        if (C.dist[c] > reach) continue;
-        float* pc = sm + NB * C.ri[c];
-        const float m1 = pc[1 - p];
-        ga[c] = add(ga[c], mul(m1, lv[c]));  // dJ/dK += mu^{n+1} o L(u^n) (kept for tile cells)
-        // mu^n = 2 mu^{n+1} - mu^{n+2} + L(K o mu^{n+1})
-        const float acc = lap5n<NB>(pc + (3 - p), rs, P.w);
-        const float v = add(sub(mul(2.0f, m1), pc[p]), acc);
-        pc[p] = v;
-        pc[2 + p] = mul(kc[c], v);
-      }
-      if (s + 1 < P.k) {
-        const float* L1 = P.lsts + (size_t)(P.ntop - s - 1) * P.cells;
-#pragma unroll
-        for (int c = 0; c < MAXC; ++c) lv[c] = __ldg(L1 + C.gi[c]);
-      }
-      __syncthreads();
-    };
-    for (int s = 0; s < P.k; s += 2) {
-      step(IC<0>{}, s);
-      if (s + 1 < P.k) step(IC<1>{}, s + 1);
-    }
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c)
-      if (C.is_tile(c)) P.gK[C.gi[c]] = ga[c];
-  } else {
-    const int nt = (int)blockDim.x;
-    const int tx0 = Rg.bx0 - Rg.rx0 - Rt.cx0, ty0 = Rg.by0 - Rg.ry0 - Rt.cy0;
-    for (int s = 0; s < P.k; ++s) {
-      const int p = s & 1;
-      const float* Ln = P.lsts + (size_t)(P.ntop - s) * P.cells;
-      RectWalk wk(Rt.W, nt);
-      for (int q = threadIdx.x; q < Rt.count; q += nt, wk.next()) {
-        const int i = (Rt.cx0 + wk.row) * RY + Rt.cy0 + wk.col;
-        float* pc = sm + NB * i;
-        const float m1 = pc[1 - p];
-        {  // gradient term of step n on the tile: dJ/dK += mu^{n+1} o L(u^n)
-          const int ox = wk.row - tx0, oy = wk.col - ty0;
-          if (ox >= 0 && ox < Rg.OX && oy >= 0 && oy < Rg.OY) {
-            const int t = oga + ox * Rg.OY + oy;
-            sm[t] = add(sm[t], mul(m1, __ldg(Ln + (size_t)(Rg.bx0 + ox) * P.Y + Rg.by0 + oy)));
-          }
+  const int nt = (int)blockDim.x;
+  const int tx0 = Rg.bx0 - Rg.rx0 - Rt.cx0, ty0 = Rg.by0 - Rg.ry0 - Rt.cy0;
+  for (int s = 0; s < P.k; ++s) {
+    const int p = s & 1;
+    const float* Ln = P.lsts + (size_t)(P.ntop - s) * P.cells;
+    RectWalk wk(Rt.W, nt);
+    for (int q = threadIdx.x; q < Rt.count; q += nt, wk.next()) {
+      const int i = (Rt.cx0 + wk.row) * RY + Rt.cy0 + wk.col;
+      float* pc = sm + NB * i;
+      const float m1 = pc[1 - p];
+      {  // gradient term of step n on the tile: dJ/dK += mu^{n+1} o L(u^n)
+        const int ox = wk.row - tx0, oy = wk.col - ty0;
+        if (ox >= 0 && ox < Rg.OX && oy >= 0 && oy < Rg.OY) {
+          const int t = oga + ox * Rg.OY + oy;
+          sm[t] = add(sm[t], mul(m1, __ldg(Ln + (size_t)(Rg.bx0 + ox) * P.Y + Rg.by0 + oy)));
         }
-        // mu^n = 2 mu^{n+1} - mu^{n+2} + L(K o mu^{n+1})
-        const float acc = lap5n<NB>(pc + (3 - p), rs, P.w);
-        const float v = add(sub(mul(2.0f, m1), pc[p]), acc);
-        pc[p] = v;
-        pc[2 + p] = mul(pc[4], v);
       }
-      __syncthreads();
+      // mu^n = 2 mu^{n+1} - mu^{n+2} + L(K o mu^{n+1})
+      const float acc = lap5n<NB>(pc + (3 - p), rs, P.w);
+      const float v = add(sub(mul(2.0f, m1), pc[p]), acc);
+      pc[p] = v;
+      pc[2 + p] = mul(pc[4], v);
     }
-    for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) { P.gK[gi] = sm[oga + t]; });
+    __syncthreads();
   }
+  for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) { P.gK[gi] = sm[oga + t]; });
   const int nw = (P.k & 1) ? 0 : 1;  // level the last step wrote
   for_tile(Rg, P.Y, [&](int t, int ri, size_t gi) {
     m1_out[gi] = sm[NB * ri + nw];
@@ -386,9 +253,7 @@ __global__ void __launch_bounds__(1024) wave_adj_tb_kernel(const float* __restri
 // are independent, so each warp interleaves two dependency chains and a step
 // of both costs one barrier.  Arithmetic and per-cell operation order are
 // those of the two kernels above.  Shared memory: the NB = 7 interleaved
-// region, then the gradient tile.  This is the general loop over the
-// rectangle (any region size); rectangles of up to 8 cells per thread run
-// the packed register-list kernel below.
+// region, then the gradient tile. 
 __global__ void __launch_bounds__(1024) wave_pair_tb_kernel(const float* __restrict__ um_in,
                                                              const float* __restrict__ u0_in,
                                                              float* __restrict__ um_out, float* __restrict__ u0_out,
@@ -463,195 +328,6 @@ __global__ void __launch_bounds__(1024) wave_pair_tb_kernel(const float* __restr
     __syncthreads();
   }
   if (adj) for_tile(Rg, Pa.Y, [&](int t, int ri, size_t gi) { Pa.gK[gi] = sm[oga + t]; });
-  const int fw = (Pf.k & 1) ? 0 : 1, aw = (Pa.k & 1) ? 0 : 1;  // levels the last steps wrote
-  for_tile(Rg, Pa.Y, [&](int t, int ri, size_t gi) {
-    const float* pc = sm + NB * ri;
-    if (fwd) {
-      um_out[gi] = pc[1 - fw];
-      u0_out[gi] = pc[fw];
-    }
-    if (adj) {
-      m1_out[gi] = pc[2 + aw];
-      m2_out[gi] = pc[3 - aw];
-    }
-  });
-}
-
-// ---- paired launch, packed: two cells per register slot --------------------
-// The paired launch's register-list form, each slot holding two cells of
-// the rectangle walked at full region width: warp w's slot c covers the 64
-// consecutive cells from 64 (w + c W) (W warps), lane l taking cells l and
-// l + 32 of them, so each half of a slot reads 32 consecutive cells (odd
-// NB-float stride: no bank conflicts).  Both chains' arithmetic runs as packed
-// pairs -- each product __ffma2_rn with a run-time -0 addend (the exactly
-// rounded product), each sum __fadd2_rn, a - b as a + (-b) -- so each half is
-// the scalar kernel's operation sequence and the results are bit-identical to
-// it.  A half outside the rectangle computes on an in-region cell (its own, or
-// the first rectangle cell past the last row) and stores nothing.
-template <int MAXP>
-struct WavePairs {
-  int ri[MAXP][2];    // region index (always inside the region)
-  int gi[MAXP][2];    // array index of a tile cell; 0 (a valid address) for the other cells
-  int dist[MAXP][2];  // distance from the tile; 1 << 20 for a half outside the rectangle
-  unsigned tile;      // bit 2c + h: half h of slot c holds a tile cell
-  __device__ bool is_tile(int c, int h) const { return (tile >> (2 * c + h)) & 1u; }
-  __device__ WavePairs(const WaveRect& Rt, const WaveRegion& Rg, int Y) {
-    const int nw = (int)blockDim.x >> 5, w = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    const int tx0 = Rg.bx0 - Rg.rx0 - Rt.cx0, ty0 = Rg.by0 - Rg.ry0;
-    const int n = Rt.NR * Rg.RY;
-    const int ri_safe = Rt.cx0 * Rg.RY + Rt.cy0;  // a rectangle cell: every neighbour inside the region
-    tile = 0;
-#pragma unroll
-    for (int c = 0; c < MAXP; ++c) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = 64 * (w + c * nw) + lane + 32 * h;  // cell of the walk: row q / RY, region column q % RY
-        ri[c][h] = ri_safe;
-        gi[c][h] = 0;
-        dist[c][h] = 1 << 20;
-        if (q < n) {
-          const int row = q / Rg.RY, col = q - row * Rg.RY;
-          ri[c][h] = (Rt.cx0 + row) * Rg.RY + col;  // rows cx0 .. cx0+NR-1: neighbours inside the region
-          if (col >= Rt.cy0 && col < Rt.cy0 + Rt.W) {
-            const int ox = row - tx0, oy = col - ty0;
-            if (ox >= 0 && ox < Rg.OX && oy >= 0 && oy < Rg.OY) {
-              gi[c][h] = (Rg.bx0 + ox) * Y + Rg.by0 + oy;
-              tile |= 1u << (2 * c + h);
-            }
-            dist[c][h] = max(max(max(-ox, ox - (Rg.OX - 1)), max(-oy, oy - (Rg.OY - 1))), 0);
-          }
-        }
-      }
-    }
-  }
-};
-
-__device__ __forceinline__ float2 wv_neg(float2 a) { return make_float2(-a.x, -a.y); }
-
-template <int MAXP>
-__global__ void __launch_bounds__(1024) wave_pair2_tb_kernel(const float* __restrict__ um_in,
-                                                              const float* __restrict__ u0_in,
-                                                              float* __restrict__ um_out, float* __restrict__ u0_out,
-                                                              const float* __restrict__ m1_in,
-                                                              const float* __restrict__ m2_in,
-                                                              float* __restrict__ m1_out, float* __restrict__ m2_out,
-                                                              const float* __restrict__ Kf, const WaveParams Pf,
-                                                              const WaveParams Pa, const float negzero) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int NB = 7;
-  const int H = max(Pf.k, Pa.k);
-  const WaveRegion Rg(Pa, H);
-  const int RY = Rg.RY, rs = NB * RY;
-  const bool fwd = Pf.k > 0, adj = Pa.k > 0;
-  for_region(Rg, [&](int i, int x, int y) {
-    const size_t gi = (size_t)x * Pa.Y + y;
-    const bool in = wave_inside(Pa, x, y);
-    float* pc = sm + NB * i;
-    cp_async4(pc + 6, Kf + gi, true);
-    if (fwd) {
-      cp_async4(pc, um_in + gi, in);
-      cp_async4(pc + 1, u0_in + gi, in);
-    }
-    if (adj) {
-      cp_async4(pc + 2, m2_in + gi, in);
-      cp_async4(pc + 3, m1_in + gi, in);
-      pc[4] = 0.0f;
-    }
-  });
-  cp_async_wait_all();
-  if (adj) for_region(Rg, [&](int i, int x, int y) { sm[NB * i + 5] = mul(sm[NB * i + 6], sm[NB * i + 3]); });
-  __syncthreads();
-  const WaveRect Rt(Pa, Rg);
-  const int srci = wave_src_index(Pf, Rg);
-  const WavePairs<MAXP> C(Rt, Rg, Pa.Y);
-  const float2 nz2 = make_float2(negzero, negzero), two2 = make_float2(2.0f, 2.0f), zero2 = make_float2(0.0f, 0.0f);
-  auto M2 = [&](float2 a, float2 b) { return __ffma2_rn(a, b, nz2); };
-  float2 wf[3], wa[3];
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    wf[t] = make_float2(Pf.w[t], Pf.w[t]);
-    wa[t] = make_float2(Pa.w[t], Pa.w[t]);
-  }
-  // the reference's 5-point sum (lap5n): x taps low to high, then y taps, from 0
-  auto lap2 = [&](const float* p0, const float* p1, const float2 (&w)[3]) {
-    auto ld = [&](int o) { return make_float2(p0[o], p1[o]); };
-    float2 acc = __fadd2_rn(zero2, M2(w[0], ld(-rs)));
-    acc = __fadd2_rn(acc, M2(w[1], ld(0)));
-    acc = __fadd2_rn(acc, M2(w[2], ld(rs)));
-    acc = __fadd2_rn(acc, M2(w[0], ld(-NB)));
-    acc = __fadd2_rn(acc, M2(w[1], ld(0)));
-    return __fadd2_rn(acc, M2(w[2], ld(NB)));
-  };
-  float2 ga[MAXP], lv[MAXP], kc[MAXP];
-#pragma unroll
-  for (int c = 0; c < MAXP; ++c) {
-    ga[c] = zero2;
-    lv[c] = zero2;
-    kc[c] = make_float2(sm[NB * C.ri[c][0] + 6], sm[NB * C.ri[c][1] + 6]);
-    if (adj) {
-      const float* L0 = Pa.lsts + (size_t)Pa.ntop * Pa.cells;
-      ga[c] = make_float2(C.is_tile(c, 0) ? Pa.gK[C.gi[c][0]] : 0.0f, C.is_tile(c, 1) ? Pa.gK[C.gi[c][1]] : 0.0f);
-      lv[c] = make_float2(__ldg(L0 + C.gi[c][0]), __ldg(L0 + C.gi[c][1]));
-    }
-  }
-  auto step = [&](auto PAR, int s) {
-    constexpr int p = decltype(PAR)::value;
-    const bool fs = s < Pf.k;
-    const float sn = (fs && srci >= 0) ? Pf.src[Pf.n0 + s] : 0.0f;
-    float* Ls = fs ? Pf.lst + (size_t)s * Pf.cells : nullptr;
-    const int freach = Pf.k - 1 - s, areach = Pa.k - 1 - s;  // negative past a chain's last step
-#pragma unroll
-    for (int c = 0; c < MAXP; ++c) {
-      float* p0 = sm + NB * C.ri[c][0];
-      float* p1 = sm + NB * C.ri[c][1];
-      const bool f0 = C.dist[c][0] <= freach, f1 = C.dist[c][1] <= freach;
-      if (f0 || f1) {  // u^{n+1} = 2 u^n - u^{n-1} + K o L(u^n) (+ source)
-        const float2 lap = lap2(p0 + (1 - p), p1 + (1 - p), wf);
-        float2 v = __fadd2_rn(M2(two2, make_float2(p0[1 - p], p1[1 - p])), wv_neg(make_float2(p0[p], p1[p])));
-        v = __fadd2_rn(v, M2(kc[c], lap));
-        if (C.ri[c][0] == srci) v.x = add(v.x, sn);
-        if (C.ri[c][1] == srci) v.y = add(v.y, sn);
-        if (f0) p0[p] = v.x;
-        if (f1) p1[p] = v.y;
-        st_global_if(Ls + C.gi[c][0], lap.x, f0 && C.is_tile(c, 0));
-        st_global_if(Ls + C.gi[c][1], lap.y, f1 && C.is_tile(c, 1));
-      }
-      const bool a0 = C.dist[c][0] <= areach, a1 = C.dist[c][1] <= areach;
-      if (a0 || a1) {  // mu^n = 2 mu^{n+1} - mu^{n+2} + L(K o mu^{n+1}); dJ/dK += mu^{n+1} o L(u^n)
-        const float2 m1 = make_float2(p0[3 - p], p1[3 - p]);
-        ga[c] = __fadd2_rn(ga[c], M2(m1, lv[c]));  // a tile half is always in reach: no other half's sum is kept
-        const float2 acc = lap2(p0 + (5 - p), p1 + (5 - p), wa);
-        const float2 v =
-            __fadd2_rn(__fadd2_rn(M2(two2, m1), wv_neg(make_float2(p0[2 + p], p1[2 + p]))), acc);
-        const float2 km = M2(kc[c], v);
-        if (a0) {
-          p0[2 + p] = v.x;
-          p0[4 + p] = km.x;
-        }
-        if (a1) {
-          p1[2 + p] = v.y;
-          p1[4 + p] = km.y;
-        }
-      }
-    }
-    if (s + 1 < Pa.k) {  // the next step's L(u^n), in flight across the barrier
-      const float* L1 = Pa.lsts + (size_t)(Pa.ntop - s - 1) * Pa.cells;
-#pragma unroll
-      for (int c = 0; c < MAXP; ++c) lv[c] = make_float2(__ldg(L1 + C.gi[c][0]), __ldg(L1 + C.gi[c][1]));
-    }
-    __syncthreads();
-  };
-  for (int s = 0; s < H; s += 2) {
-    step(IC<0>{}, s);
-    if (s + 1 < H) step(IC<1>{}, s + 1);
-  }
-  if (adj) {
-#pragma unroll
-    for (int c = 0; c < MAXP; ++c) {
-      if (C.is_tile(c, 0)) Pa.gK[C.gi[c][0]] = ga[c].x;
-      if (C.is_tile(c, 1)) Pa.gK[C.gi[c][1]] = ga[c].y;
-    }
-  }
   const int fw = (Pf.k & 1) ? 0 : 1, aw = (Pa.k & 1) ? 0 : 1;  // levels the last steps wrote
   for_tile(Rg, Pa.Y, [&](int t, int ri, size_t gi) {
     const float* pc = sm + NB * ri;

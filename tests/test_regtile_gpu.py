@@ -117,3 +117,27 @@ def test_batched_wave_window_edges(k, nsteps):
         st = fdm.wave_forward(np.full(u[i].shape, K[i], np.float32), u[i], None, -1, nsteps, dx[i])
         assert np.array_equal(now[i].cpu().numpy()[:, :, 0, 0], st[-1]), boxes[i]
         assert np.array_equal(prev[i].cpu().numpy()[:, :, 0, 0], st[-2]), boxes[i]
+
+
+@pytest.mark.parametrize("X,Y,g,N,k,every,src", [(12, 12, 1, 5, 0, None, None), (68, 132, 1, 21, 0, 7, (5, 60)),
+                                                 (69, 133, 1, 21, 5, None, (30, 131)), (70, 203, 2, 17, 0, 6, (1, 1)),
+                                                 (204, 67, 1, 30, 12, 12, (100, 33))])
+def test_wave_window_edges(X, Y, g, N, k, every, src):
+    """Forward and adjoint windows at even and odd sides (paired and single columns),
+    one window, several, a source on an edge and on a ghost; against the oracle."""
+    rng = np.random.default_rng(X + Y)
+    dx = 1.0 / (X - 3)
+    K = (0.1 * dx * dx * (1.0 + rng.random((X, Y, 1, 1)))).astype(np.float32)
+    u0 = rng.standard_normal((X, Y, 1, 1)).astype(np.float32)
+    grad = rng.standard_normal((X, Y, 1, 1)).astype(np.float32)
+    s = (dx * dx * rng.random(N)).astype(np.float32)
+    solver = P.WaveSolver((X, Y, 1), dx, N, src=torch.from_numpy(s).cuda() if src else None, src_cell=src, ghost_cells=g,
+                          steps_per_pass=k, checkpoint_every=every)
+    Kd = torch.from_numpy(K).cuda()
+    uN = solver.forward(Kd, torch.from_numpy(u0).cuda())
+    gK, gu = solver.backward(Kd, torch.from_numpy(grad).cuda())
+    st = fdm.wave_forward(K, u0, s, src[0] * Y + src[1] if src else -1, N, dx, ghost=g)
+    rgK, mu0, mu1 = fdm.wave_adjoint(K, st, grad, dx, ghost=g)
+    assert np.array_equal(uN.cpu().numpy()[:, :, 0, 0], st[-1])
+    assert np.array_equal(gK.cpu().numpy()[:, :, 0, 0], rgK)
+    assert np.array_equal(gu.cpu().numpy()[:, :, 0, 0], mu0 - mu1)
