@@ -832,6 +832,17 @@ void pick_tile_2d(int X, int Y, int* tbx, int* tby) {
   }
 }
 
+// The register-tile passes of the differentiable heat (order 2, every face filled,
+// boxes of 8 cells a side or more); the shared-memory kernels take the rest.
+RTPlan heat_field_plan(const Geo& G, const PdeBCRules& rules, bool adjoint, int nsteps, int steps_per_pass) {
+  if (g_dispatch == PDE_DISPATCH_GENERIC) {
+    RTPlan no;
+    no.ok = false;
+    return no;
+  }
+  return rt_heat_field_plan(G, rules, adjoint, nsteps, steps_per_pass, g_tile2d[0], g_tile2d[1]);
+}
+
 // Shared checks and launch geometry of the differentiable heat entry points.
 int heat_diff_setup(const PdeGrid* grid, const PdeBCRules* rules, int steps_per_pass, int nsteps, Geo* G,
                     HAParams* P, int* kk) {
@@ -926,17 +937,24 @@ int heat_forward_run(const float* alpha, const float* u_in, float* u_out, float*
   P.ramp = rules->has_ramp ? 1 : 0;
   P.t0 = t0;
   P.tstep = tstep;
+  const RTPlan L = heat_field_plan(G, *rules, false, nsteps, steps_per_pass);
+  if (L.ok) k = L.k;
   const int npasses = (nsteps + k - 1) / k;
   const bool alias = (u_out == u_in);
   const float* src = u_in;
   float* dst = alias ? work : ((npasses % 2 == 1) ? u_out : work);
   int done = 0;
   for (int p = 0; p < npasses; ++p) {
-    P.k = (nsteps - done < k) ? (nsteps - done) : k;
+    P.k = (nsteps - done + npasses - p - 1) / (npasses - p);  // passes of even depth
     P.lst = lstates ? lstates + (size_t)done * P.cells : nullptr;
     P.n0 = n0 + done;
-    kern<<<tiles, threads, smem, st>>>(src, dst, P, *rules);
-    rc = launch_status();
+    if (L.ok) {
+      const HeatFieldPass H{P.X, P.Y, P.g, P.k, {P.w[0], P.w[1]}, dt, alpha, src, dst, P.lst, nullptr, nullptr, t0, tstep, P.n0};
+      rc = rt_heat_field_pass(L, H, *rules, st);
+    } else {
+      kern<<<tiles, threads, smem, st>>>(src, dst, P, *rules);
+      rc = launch_status();
+    }
     if (rc) return rc;
     done += P.k;
     src = dst;
@@ -982,16 +1000,24 @@ int pde_heat_adjoint(const float* alpha, const float* lam_in, float* lam_out, co
   P.dt = dt;
   P.lsts = lstates;
   P.galpha = grad_alpha;
+  const RTPlan L = heat_field_plan(G, *rules, true, nsteps, steps_per_pass);
+  if (L.ok) k = L.k;
   const int npasses = (nsteps + k - 1) / k;
   const bool alias = (lam_out == lam_in);
   const float* src = lam_in;
   float* dst = alias ? work : ((npasses % 2 == 1) ? lam_out : work);
   int done = 0;
   for (int p = 0; p < npasses; ++p) {
-    P.k = (nsteps - done < k) ? (nsteps - done) : k;
+    P.k = (nsteps - done + npasses - p - 1) / (npasses - p);  // passes of even depth
     P.ntop = nsteps - 1 - done;
-    kern<<<tiles, threads, smem, st>>>(src, dst, P, *rules);
-    rc = launch_status();
+    if (L.ok) {
+      const HeatFieldPass H{P.X, P.Y, P.g, P.k, {P.w[0], P.w[1]}, dt, alpha, src, dst, nullptr,
+                            lstates + (size_t)P.ntop * P.cells, grad_alpha, 0.0, 0.0, 0};
+      rc = rt_heat_field_pass(L, H, *rules, st);
+    } else {
+      kern<<<tiles, threads, smem, st>>>(src, dst, P, *rules);
+      rc = launch_status();
+    }
     if (rc) return rc;
     done += P.k;
     src = dst;

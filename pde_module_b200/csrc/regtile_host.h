@@ -88,4 +88,19 @@ struct WaveAdj {
 RTPlan rt_wave_plan(const WaveRun& J, bool fwd, bool adj, int nsteps, int k_req, int tile_x, int tile_y);
 int rt_wave_pass(const RTPlan& L, const WaveRun& J, const WaveFwd* f, const WaveAdj* a, cudaStream_t st);
 
+// Passes of the differentiable heat rollout of order 2 (heat_adj_rt.cuh).
+struct HeatFieldPass {
+  int X, Y, g, k;
+  float w[2], dt;
+  const float *alpha, *in;
+  float *out, *lst;
+  const float* lsts;
+  float* galpha;  // set: an adjoint pass
+  double t0, tstep;
+  int n0;
+};
+RTPlan rt_heat_field_plan(const Geo& G, const PdeBCRules& rules, bool adjoint, int nsteps, int k_req, int tile_x,
+                          int tile_y);
+int rt_heat_field_pass(const RTPlan& L, const HeatFieldPass& H, const PdeBCRules& rules, cudaStream_t st);
+
 }  // namespace pde

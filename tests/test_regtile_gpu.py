@@ -141,3 +141,31 @@ def test_wave_window_edges(X, Y, g, N, k, every, src):
     assert np.array_equal(uN.cpu().numpy()[:, :, 0, 0], st[-1])
     assert np.array_equal(gK.cpu().numpy()[:, :, 0, 0], rgK)
     assert np.array_equal(gu.cpu().numpy()[:, :, 0, 0], mu0 - mu1)
+
+
+@pytest.mark.parametrize("sides", [(8, 8), (9, 33), (64, 64), (65, 130), (203, 71)])
+@pytest.mark.parametrize("spec", [DIRICHLET, MIXED, NEUMANN])
+def test_heat_gradient_window_edges(sides, spec):
+    """Forward with a diffusivity field and its adjoint: the transposed boundary fill at
+    corners, one window and several, short passes; against the oracle."""
+    X, Y = sides[0] + 2, sides[1] + 2
+    rng = np.random.default_rng(X * Y)
+    dx = 1.0 / sides[0]
+    dt = 0.2 * dx * dx
+    alpha = (0.5 + 0.5 * rng.random((X, Y, 1, 1))).astype(np.float32)
+    u0 = rng.random((X, Y, 1, 1)).astype(np.float32)
+    lam = rng.standard_normal((X, Y, 1, 1)).astype(np.float32)
+    bc = P.GridBoundary(torch.from_numpy(u0).cuda(), dx, 1)
+    for name, typ, val, comps in spec:
+        bc.set_BC(name, val, typ, comps)
+    groups = fdm.standard_groups((X, Y, 1), 1, spec)
+    for N, k, every in ((1, 0, None), (14, 4, 6), (21, 0, None)):
+        solver = P.HeatSolver(bc, dx, dt, N, steps_per_pass=k, checkpoint_every=every)
+        a = torch.from_numpy(alpha).cuda()
+        uN = solver.forward(a, torch.from_numpy(u0).cuda())
+        ga, gu = solver.backward(a, torch.from_numpy(lam).cuda())
+        ref, S = fdm.heat_forward_field(alpha, u0, groups, dx, 1, dt, N)
+        rga, rgu = fdm.heat_adjoint(alpha, S, lam, groups, dx, 1, dt)
+        assert np.array_equal(uN.cpu().numpy(), ref), N
+        assert np.array_equal(ga.cpu().numpy(), rga), N
+        assert np.array_equal(gu.cpu().numpy(), rgu), N
