@@ -135,45 +135,114 @@ struct Shell {
   }
 };
 
-// Surface fill of the one-step 3D heat rollout, first pass: every cell outside
-// the stencil box [g, n-g)^3 takes its boundary-filled value u2 (bc_eval) in u
-// (in place: a ghost's value reads its partner two cells inward, never another
-// ghost cell, and deeper ghosts keep their value) and, when out is set, in the
-// step's output (the first step seeds the constant deeper ghosts there; the last
-// leaves the result's ghosts; steps between skip it, their output's ghosts
-// being recomputed before anything reads them).
-__global__ void __launch_bounds__(256) heat_fill_ghosts_kernel(float* __restrict__ u, float* __restrict__ out, Geo G,
-                                                               int N, const PdeBCRules Rl, Shell S) {
-  GlobalAcc U{u, G.cstride[0], G.cstride[1], N};
-  const long long total = S.off[6] * N;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long i = t / N;
-    const int v = (int)(t - i * N);
-    int c[3];
-    S.cell(i, c);
-    const float u2 = bc_eval(G, Rl, U, c[0], c[1], c[2], v);
-    const long long k = ((long long)c[0] * G.n[1] + c[1]) * G.n[2] + c[2];
-    u[k * N + v] = u2;
-    if (out) out[k * N + v] = u2;
+// The boundary rules of a 3D scalar field as a table: the ghost across face f (x low,
+// x high, y low, ...) of a node of classes (a, b) along the two other axes is
+// s * partner + c (s = 0: no group fills it), nodes of class K take their value where
+// `set`.
+struct Fill3 {
+  float2 ghost[6][9];
+  float2 node[27];
+};
+
+// What the fill makes of one box cell, in place: a ghost's partner is the cell next to
+// the node, so the cell writes the ghosts it is the partner of, from its own value,
+// then its own boundary value if it is a node.  No cell reads another: one pass.
+__device__ __forceinline__ void fill3_cell(float* u, const Geo& G, const Fill3& F, int x, int y, int z, float v) {
+  const int g = G.g;
+  const int c[3] = {x, y, z}, n[3] = {(int)G.n[0], (int)G.n[1], (int)G.n[2]};
+  const long long stride[3] = {G.cstride[0], G.cstride[1], 1};
+  int k[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) k[a] = c[a] == g ? 0 : (c[a] == n[a] - 1 - g ? 2 : 1);
+  float* o = u + x * stride[0] + y * stride[1] + z;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int q0 = a == 0 ? 1 : 0, q1 = a == 2 ? 1 : 2, cls = 3 * k[q0] + k[q1];
+    if (c[a] == g + 1) {
+      const float2 t = F.ghost[2 * a][cls];
+      if (t.x != 0.0f) o[-2 * stride[a]] = fmaf(t.x, v, t.y);  // one rounding, as ghost_value (s is +-1)
+    }
+    if (c[a] == n[a] - 2 - g) {
+      const float2 t = F.ghost[2 * a + 1][cls];
+      if (t.x != 0.0f) o[2 * stride[a]] = fmaf(t.x, v, t.y);
+    }
+  }
+  const float2 m = F.node[9 * k[0] + 3 * k[1] + k[2]];
+  if (m.y != 0.0f) *o = m.x;
+}
+
+// Coordinates with a part in the fill along an axis of `ext` box cells: the two first
+// and the two last (all when there are no more than four).
+struct Fill3Axis {
+  int n, g, faces, inner;
+  __host__ __device__ Fill3Axis(int n_, int g_) : n(n_), g(g_) {
+    const int ext = n - 2 * g;
+    faces = ext < 4 ? ext : 4;
+    inner = ext - faces;
+  }
+  __host__ __device__ int face(int i) const { return i < 2 ? g + i : n - 1 - g - (faces - 1 - i); }
+};
+
+// Boundary fill of the one-step 3D heat rollout's source: a warp per 128 cells of a row
+// (x, y) of the faces along X and Y, then a thread per remaining row for its cells at the faces along
+// Z.  Bound by latency (a few scattered sectors per row): loads come before
+// stores and rows are cut in pieces.  Two kernels over the shell's cells, evaluating the
+// rules for each, took 21 us of a 57 us step on 256 x 192 x 320; this one takes about
+// 6, and the step 41.  Writing the fill from the streaming kernel that computes the
+// partner was slower (150 us: the calls spill its register queue).
+__global__ void __launch_bounds__(256) heat_fill3_kernel(float* __restrict__ u, Geo G,
+                                                         const __grid_constant__ Fill3 F, int row_blocks) {
+  pdl_launch_dependents();
+  const Fill3Axis AX((int)G.n[0], G.g), AY((int)G.n[1], G.g), AZ((int)G.n[2], G.g);
+  const int ey = AY.faces + AY.inner, ez = AZ.faces + AZ.inner;
+  pdl_wait();  // the previous step's output (this step's source) is complete
+  if ((int)blockIdx.x < row_blocks) {
+    const int parts = (ez + 127) / 128, w = (int)blockIdx.x * 8 + ((int)threadIdx.x >> 5);
+    const int row = w / parts, xrows = AX.faces * ey;
+    int x, y;
+    if (row < xrows) {
+      x = AX.face(row / ey);
+      y = G.g + row % ey;
+    } else {
+      const int q = row - xrows;
+      if (q >= AX.inner * AY.faces) return;
+      x = G.g + 2 + q / AY.faces;
+      y = AY.face(q % AY.faces);
+    }
+    const float* p = u + x * G.cstride[0] + y * G.cstride[1] + G.g;
+    const int z0 = (w - row * parts) * 128 + ((int)threadIdx.x & 31);
+    float v[4];  // loaded before any store: the compiler cannot tell the cells apart
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = z0 + 32 * i < ez ? p[z0 + 32 * i] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (z0 + 32 * i < ez) fill3_cell(u, G, F, x, y, G.g + z0 + 32 * i, v[i]);
+  } else {
+    const int q = ((int)blockIdx.x - row_blocks) * 256 + (int)threadIdx.x;
+    if (q >= AX.inner * AY.inner) return;
+    const int x = G.g + 2 + q / AY.inner, y = G.g + 2 + q % AY.inner;
+    const float* p = u + x * G.cstride[0] + y * G.cstride[1];
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = i < AZ.faces ? p[AZ.face(i)] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < AZ.faces) fill3_cell(u, G, F, x, y, AZ.face(i), v[i]);
   }
 }
 
-// Second pass: the node layers (coordinate g or n-1-g inside the stencil box)
-// take their Dirichlet values in u, after every ghost has read its partner's
-// pre-boundary value.
-__global__ void __launch_bounds__(256) heat_fill_nodes_kernel(float* __restrict__ u, Geo G, int N,
-                                                              const PdeBCRules Rl, Shell S) {
-  GlobalAcc U{u, G.cstride[0], G.cstride[1], N};
-  const long long total = S.off[6] * N;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long i = t / N;
-    const int v = (int)(t - i * N);
+// The g outer layers of src into dst (a buffer's first use; the last step's ghosts, as
+// its source had them).
+__global__ void __launch_bounds__(256) heat_copy_shell_kernel(const float* __restrict__ src, float* __restrict__ dst,
+                                                              Geo G, Shell S) {
+  pdl_launch_dependents();
+  pdl_wait();
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < S.off[6];
+       i += (long long)gridDim.x * blockDim.x) {
     int c[3];
     S.cell(i, c);
-    const float u2 = bc_eval(G, Rl, U, c[0], c[1], c[2], v);
-    u[(((long long)c[0] * G.n[1] + c[1]) * G.n[2] + c[2]) * N + v] = u2;
+    const long long k = ((long long)c[0] * G.n[1] + c[1]) * G.n[2] + c[2];
+    dst[k] = src[k];
   }
 }
 

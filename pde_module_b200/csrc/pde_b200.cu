@@ -136,6 +136,7 @@ int launch_stream3d_k(const float* in, float* out, const Geo& G, const Weights& 
       for (int t = R + 1; t < 2 * R + 1; ++t) FW.a[t - R - 1] = (float)(alpha_d * Wt.wd[t]);
     }
   }
+  if constexpr (OP == OP_HEAT) return launch_pdl(kern, (int)blocks, C::THREADS, C::SMEM, st, m, P, FW);
   kern<<<(unsigned)blocks, C::THREADS, C::SMEM, st>>>(m, P, FW);
   return launch_status();
 }
@@ -545,15 +546,20 @@ float host_ramp_value(const PdeBCGroupParam& B, double t0, double tstep, long lo
   return r * B.value;
 }
 
-// One step per pass on the TMA streaming kernel (OP_HEAT) after a surface fill:
-// scalar 3D fields whose shape takes the double-row map (even Y and Z, 16-byte
-// plane pitch, even g - R) and whose index fits the 1D view.
-bool heat_split_shape(const Geo& G, int ncomp) {
+// One step per pass on the TMA streaming kernel: scalar 3D fields whose index fits
+// the 1D view.
+bool heat_stream_shape(const Geo& G, int ncomp) {
   if (g_dispatch == PDE_DISPATCH_GENERIC || G.ndims != 3 || ncomp != 1) return false;
   const int R = G.order / 2;
   const int64_t slack = 64LL * G.n[2] + 1024;
-  return pick_map<1>(G, R) == MAP_PAIRS && G.n[0] * G.n[1] * G.n[2] + slack < (1LL << 31) && G.g >= R &&
+  return G.n[0] * G.n[1] * G.n[2] + slack < (1LL << 31) && G.g >= R &&
          G.ext[0] >= 3 && G.ext[1] >= 3 && G.ext[2] >= 3;
+}
+
+// Those whose shape takes the double-row map (even Y and Z, 16-byte plane pitch,
+// even g - R).
+bool heat_split_shape(const Geo& G, int ncomp) {
+  return heat_stream_shape(G, ncomp) && pick_map<1>(G, G.order / 2) == MAP_PAIRS;
 }
 
 // Steps per pass of the fused rollout for a request (0 = choose): 2D grids 8;
@@ -568,11 +574,57 @@ int heat_depth(const Geo& G, int ncomp, int steps_per_pass) {
   return k > heat3d_kmax(ncomp) ? heat3d_kmax(ncomp) : k;
 }
 
-// The one-step streaming 3D rollout: per step a surface fill of the source
-// buffer (ghosts into the source and the output, then nodes into the source)
-// and the OP_HEAT streaming kernel over the stencil box.  The caller's input is
-// first copied into a buffer of this call (the fill writes in place), chosen so
-// the last step lands in u_out; with u_out == u_in the rollout runs in place.
+// The boundary rules as the fill's table.
+Fill3 fill_table(const PdeBCRules& R) {
+  Fill3 F;
+  for (int f = 0; f < 6; ++f)
+    for (int cls = 0; cls < 9; ++cls) {
+      const int a = f >> 1, q0 = a == 0 ? 1 : 0, q1 = a == 2 ? 1 : 2;
+      int k[3];
+      k[a] = (f & 1) ? 2 : 0;
+      k[q0] = cls / 3;
+      k[q1] = cls % 3;
+      const int gi = R.ghost_group[9 * k[0] + 3 * k[1] + k[2]][a][0];
+      float2 t = make_float2(0.0f, 0.0f);
+      if (gi >= 0) {
+        const float v = R.group[gi].value;
+        const int inc = (f & 1) ? -1 : 1;
+        const float step = (float)(-2 * inc) * R.dx32;  // each product rounded, as ghost_value has it
+        t = R.group[gi].type == PDE_BC_DIRICHLET ? make_float2(-1.0f, 2.0f * v) : make_float2(1.0f, step * v);
+      }
+      F.ghost[f][cls] = t;
+    }
+  for (int K = 0; K < 27; ++K) {
+    const int gi = R.node_group[K];
+    F.node[K] = gi >= 0 && (R.group[gi].comp_mask & 1u) ? make_float2(R.group[gi].value, 1.0f) : make_float2(0.0f, 0.0f);
+  }
+  return F;
+}
+
+// One step of the streaming rollout.  Tiles by plane addressing (pick_map): the
+// double-row map's, or the row maps' (one copy per row) for odd sides.
+int launch_heat_stream(const float* src, float* dst, const Geo& G, const Weights& W, float alpha, float dt,
+                       cudaStream_t st) {
+  const int map = pick_map<1>(G, G.order / 2);
+  if (G.order == 2) {
+    if (map == MAP_PAIRS)
+      return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+    if (map == MAP_ROWS_PP0)
+      return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_ROWS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+    return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_ROWS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+  }
+  if (map == MAP_PAIRS)
+    return launch_stream3d_k<2, OP_HEAT, 1, 128, 16, 4, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+  if (map == MAP_ROWS_PP0)
+    return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_ROWS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+  return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_ROWS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+}
+
+// The one-step streaming 3D rollout: per step the fill of the source's boundary in
+// place (heat_fill3_kernel) and the OP_HEAT streaming kernel over the stencil box, each
+// a dependent launch of the one before.  The caller's input is first copied into a
+// buffer of this call (the fill writes in place), chosen so the last step lands in
+// u_out; with u_out == u_in the rollout runs in place.
 // input_scratch: the caller lets the input be overwritten, so step 0 fills it
 // in place and the steps alternate between work and u_out, ending in u_out.
 int heat3d_split_run(const float* u_in, float* u_out, float* work, const Geo& G, const Weights& W,
@@ -594,29 +646,31 @@ int heat3d_split_run(const float* u_in, float* u_out, float* work, const Geo& G,
     dst = (first == work) ? u_out : work;
   }
   const int n[3] = {(int)G.n[0], (int)G.n[1], (int)G.n[2]};
-  Shell gs, ns;
+  Shell gs;
   gs.init(n, 0, G.g);
-  ns.init(n, G.g, 1);
   const int sms = sm_count();
-  auto blocks_for = [&](long long cells) {
-    const long long b = (cells + 255) / 256;
-    return (int)(b < 8LL * sms ? (b > 0 ? b : 1) : 8LL * sms);
-  };
+  const Fill3Axis AX(n[0], G.g), AY(n[1], G.g);
+  const int rows = AX.faces * (AY.faces + AY.inner) + AX.inner * AY.faces;
+  const int parts = (n[2] - 2 * G.g + 127) / 128;  // warps per row
+  const int row_blocks = (rows * parts + 7) / 8, fill_blocks = row_blocks + (AX.inner * AY.inner + 255) / 256;
+  const long long shell_blocks = (gs.off[6] + 255) / 256 < 8LL * sms ? (gs.off[6] + 255) / 256 : 8LL * sms;
   PdeBCRules Rs = *rules;
+  Fill3 F = fill_table(Rs);
   for (int s = 0; s < nsteps; ++s) {
-    if (rules->has_ramp)
+    if (rules->has_ramp) {
       for (int i = 0; i < rules->ngroups; ++i)
         if (rules->group[i].func == PDE_BC_FUNC_RAMP)
           Rs.group[i].value = host_ramp_value(rules->group[i], t0, tstep, (long long)n0 + s);
-    heat_fill_ghosts_kernel<<<blocks_for(gs.off[6]), 256, 0, st>>>(src, (s == 0 || s == nsteps - 1) ? dst : nullptr,
-                                                                    G, 1, Rs, gs);
-    heat_fill_nodes_kernel<<<blocks_for(ns.off[6]), 256, 0, st>>>(src, G, 1, Rs, ns);
-    int rc = launch_status();
+      F = fill_table(Rs);
+    }
+    int rc = launch_pdl(heat_fill3_kernel, fill_blocks, 256, 0, st, src, G, F, row_blocks);
     if (rc) return rc;
-    if (G.order == 2)
-      rc = launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
-    else
-      rc = launch_stream3d_k<2, OP_HEAT, 1, 128, 16, 4, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+    if (s == 0 || s == nsteps - 1 || (s == 1 && input_scratch)) {
+      rc = launch_pdl(heat_copy_shell_kernel, (int)(shell_blocks > 0 ? shell_blocks : 1), 256, 0, st,
+                      static_cast<const float*>(src), dst, G, gs);
+      if (rc) return rc;
+    }
+    rc = launch_heat_stream(src, dst, G, W, alpha, dt, st);
     if (rc) return rc;
     float* t = src;
     src = dst;
@@ -656,7 +710,9 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
   }
   int k = heat_depth(G, ncomp, steps_per_pass);
   if (k > nsteps) k = nsteps;
-  if (s3d && k == 1 && heat_split_shape(G, ncomp) && aligned16(u_in) && aligned16(u_out) && aligned16(work))
+  // a depth left open streams one step per pass on any shape (odd sides too, where the
+  // row maps take 47 us a step on 255 x 191 x 319 against 163 of the blocked kernel)
+  if (s3d && (steps_per_pass == 0 || k == 1) && heat_stream_shape(G, ncomp) && aligned16(u_in) && aligned16(u_out) && aligned16(work))
     return heat3d_split_run(u_in, u_out, work, G, W, rules, alpha, dt, nsteps, t0, tstep, n0, input_scratch, st);
   const int npasses = (nsteps + k - 1) / k;
   // buffer sequence: the last pass writes u_out.

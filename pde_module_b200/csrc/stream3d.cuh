@@ -369,6 +369,10 @@ __global__ void __launch_bounds__(S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MOD
     }
     mbar_fence_init();
   }
+  if constexpr (OP == OP_HEAT) {
+    pdl_launch_dependents();  // the next step's fill may be scheduled; it waits for this kernel
+    pdl_wait();               // the fill of this step's source is complete
+  }
   __syncthreads();
 
   if (tid >= C::NCONS) {

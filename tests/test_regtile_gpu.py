@@ -169,3 +169,25 @@ def test_heat_gradient_window_edges(sides, spec):
         assert np.array_equal(uN.cpu().numpy(), ref), N
         assert np.array_equal(ga.cpu().numpy(), rga), N
         assert np.array_equal(gu.cpu().numpy(), rgu), N
+
+
+@pytest.mark.parametrize("shape,order", [((9, 8, 10), 2), ((5, 7, 6), 2), ((20, 33, 47), 2), ((34, 30, 132), 2),
+                                         ((6, 137, 135), 2), ((20, 33, 47), 4), ((34, 30, 36), 4)])
+@pytest.mark.parametrize("spec", [DIRICHLET, [("ALL", 2, 0.3, (0,)), ("-X", 1, 0.25, (0,)), ("+Z", 1, -1.0, (0,))],
+                                  [("-Y", 1, 0.4, (0,)), ("+X", 2, -0.3, (0,))]])
+def test_heat3d_streaming_fill(shape, order, spec):
+    """The one-step 3D path on even and odd sides (its row maps), from three interior
+    cells a side; the single-pass fill at faces, edges, corners and unfilled faces."""
+    g = order // 2
+    dx = 1.0 / shape[0]
+    dt = 0.1 * dx * dx
+    u0 = np.random.default_rng(sum(shape)).random(shape + (1,)).astype(np.float32)
+    ud = torch.from_numpy(u0).cuda()
+    bc = P.GridBoundary(ud, dx, g)
+    for name, typ, val, comps in spec:
+        bc.set_BC(name, val, typ, comps)
+    groups = fdm.standard_groups(shape, g, spec)
+    for steps in (1, 2, 5):
+        got = P.HeatRollout(bc, dx, 0.9, dt, order=order)(ud, steps).cpu().numpy()
+        assert np.array_equal(got, fdm.heat_rollout(u0, groups, dx, g, 0.9, dt, steps, order)), steps
+    assert np.array_equal(ud.cpu().numpy(), u0)
