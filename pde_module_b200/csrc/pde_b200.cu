@@ -1516,17 +1516,26 @@ int pde_wc_rk2(const float* m_in, const float* rho_in, float* m_out, float* rho_
   P.X = (int)G.n[0];
   P.Y = (int)G.n[1];
   P.g = G.g;
-  // automatic shape: 32x32 tiles; 16x16 when those leave SMs idle, 64x32 when
-  // there are several per SM (fewer halo cells per tile cell)
-  const long long t32 = (long long)((P.X + 31) / 32) * ((P.Y + 31) / 32);
-  P.TBX = P.TBY = 32;
-  if (t32 < sm_count()) P.TBX = P.TBY = 16;
-  else if (t32 >= 4LL * sm_count()) P.TBX = 64;
+  // Automatic shape.  One cell of the region per thread is the fastest step as long as
+  // the tiles are resident together (tiles of 17 fill the 640 threads; two such blocks
+  // fit an SM): the smallest tile of at most one per SM, then 17 (us per step with 17 /
+  // 24 / 32: 257^2 nodes 11.4 / 13.0 / 19.9).  Beyond that halo cells cost more than
+  // waiting: 24 while three blocks per SM hold them all (400^2: 18.4 / 18.9 / 21.7,
+  // 300^2: 15.1 / 14.9 / 18.0), then 32 (600^2: 35.1 / 30.0 / 28.7; 64x32 is no faster).
+  auto tiles_of = [&](int side) { return (long long)((P.X + side - 1) / side) * ((P.Y + side - 1) / side); };
+  const long long sms = sm_count();
+  constexpr int SIDE1 = 17;  // (17 + 2 WC_HALO)^2 <= WC_THREADS
+  int side = 8, threads = 512;
+  while (side < SIDE1 && tiles_of(side) > sms) ++side;
+  if (tiles_of(side) > 2 * sms) side = tiles_of(24) <= 3 * sms ? 24 : 32;
+  if (side <= SIDE1) threads = ((side + 2 * WC_HALO) * (side + 2 * WC_HALO) + 31) / 32 * 32;
+  P.TBX = P.TBY = side;
   if (g_tile2d[0] > 0) {  // pde_set_launch_2d
     P.TBX = g_tile2d[0];
     P.TBY = g_tile2d[1];
+    threads = 512;
   }
-  const int threads = (g_threads2d == 256 || g_threads2d == 512) ? g_threads2d : 512;
+  if (g_threads2d == 256 || g_threads2d == 512) threads = g_threads2d;
   P.tiles_y = (P.Y + P.TBY - 1) / P.TBY;
   P.RC = (P.TBX + 2 * WC_HALO) * (P.TBY + 2 * WC_HALO);
   const size_t smem = (size_t)10 * P.RC * sizeof(float);
@@ -1553,8 +1562,7 @@ int pde_wc_rk2(const float* m_in, const float* rho_in, float* m_out, float* rho_
   for (int s = 0; s < nsteps; ++s) {
     float* dm = to_out ? m_out : wm;
     float* dr = to_out ? rho_out : wr;
-    wc_rk2_kernel<<<tiles, threads, smem, st>>>(sm_, sr, dm, dr, P, *u_rules, *rho_rules);
-    const int rc = launch_status();
+    const int rc = launch_pdl(wc_rk2_kernel, tiles, threads, smem, st, sm_, sr, dm, dr, P, *u_rules, *rho_rules);
     if (rc) return rc;
     sm_ = dm;
     sr = dr;

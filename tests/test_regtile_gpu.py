@@ -191,3 +191,17 @@ def test_heat3d_streaming_fill(shape, order, spec):
         got = P.HeatRollout(bc, dx, 0.9, dt, order=order)(ud, steps).cpu().numpy()
         assert np.array_equal(got, fdm.heat_rollout(u0, groups, dx, g, 0.9, dt, steps, order)), steps
     assert np.array_equal(ud.cpu().numpy(), u0)
+
+
+@pytest.mark.parametrize("shape", [(7, 9), (95, 101), (203, 204), (242, 290), (331, 403), (520, 640)])
+def test_weakly_compressible_tile_rule(shape):
+    """The automatic tiles of the weakly compressible step at each of its sides (8, one
+    per SM, 17, 24, 32) and their remainders, on a momentum that is only 4-byte aligned."""
+    from oracle import acm
+    from tests.test_wc_gpu import _case
+    m, rho, md, rd, u_bc, r_bc, ug, rg, dx, nu, c2, rho0, eps, dt = _case(shape + (1,), 11)
+    odd = torch.empty(md.numel() + 1, device="cuda")[1:].view(md.shape).copy_(md)
+    got_m, got_r = P.WeaklyCompressibleRK2(u_bc, r_bc, dx, nu, c2, rho0, eps, dt)(odd, rd, 2)
+    ref_m, ref_r = acm.wc_rk2(m, rho, ug, rg, dx, 1, nu, eps, c2, rho0, dt, 2)
+    assert np.array_equal(got_m.cpu().numpy(), ref_m)
+    assert np.array_equal(got_r.cpu().numpy(), ref_r)
