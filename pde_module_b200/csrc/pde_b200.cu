@@ -123,8 +123,13 @@ int launch_stream3d_k(const float* in, float* out, const Geo& G, const Weights& 
     if (!encode_3d(&m, in, 2 * zc, (uint64_t)G.n[1] / 2, (uint64_t)G.n[0], 8 * zc, 4 * zc * (uint64_t)G.n[1],
                    (uint32_t)C::W, (uint32_t)(C::ROWS / 2)))
       return PDE_ERR_CUDA;
-  } else if (!encode_1d(&m, in, (uint64_t)total, (uint32_t)C::W)) {
-    return PDE_ERR_CUDA;
+  } else {
+    const uint64_t zc = (uint64_t)G.n[2] * CIN, quads = (uint64_t)(G.n[0] * G.n[1] / 4);
+    P.in = in;
+    P.total = (int)total;
+    P.full_rows = (int)(4 * quads);
+    if (!encode_3d(&m, in, 4 * zc, quads, 1, 16 * zc, 16 * zc * quads, (uint32_t)C::W, (uint32_t)C::QROWS))
+      return PDE_ERR_CUDA;
   }
   FastW FW{};
   if (MODE == MODE_FAST) {
@@ -143,7 +148,7 @@ int launch_stream3d_k(const float* in, float* out, const Geo& G, const Weights& 
 
 // Plane addressing for a grid: double-row boxes when the array's row pairs and
 // planes have 16-byte multiple pitches and the tile rows start on even rows;
-// else one copy per row (lead fixed across planes when the plane pitch is a
+// else quadruple rows (lead fixed across planes when the plane pitch is a
 // multiple of 4 floats).
 template <int CIN>
 int pick_map(const Geo& G, int R) {
@@ -151,25 +156,23 @@ int pick_map(const Geo& G, int R) {
   if ((G.n[1] % 2) == 0 && (zc % 2) == 0 && ((G.n[1] * zc) % 4) == 0 && ((G.g - R) % 2) == 0 &&
       G.n[1] / 2 < (1LL << 31) && 2 * zc < (1LL << 31))
     return MAP_PAIRS;
-  return ((G.n[1] * zc) & 3) == 0 ? MAP_ROWS_PP0 : MAP_ROWS_GEN;
+  return ((G.n[1] * zc) & 3) == 0 ? MAP_QUADS_PP0 : MAP_QUADS_GEN;
+}
+
+template <int R, int OP, int CIN, int TZ, int TY, int YPT, int PREF, int MAPK>
+int launch_stream3d(const float* in, float* out, const Geo& G, const Weights& Wt, float alpha, int mode,
+                    cudaStream_t st) {
+  if (mode == PDE_MODE_FAST)
+    return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MODE_FAST>(in, out, G, Wt, alpha, alpha, st);
+  return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MODE_EXACT>(in, out, G, Wt, alpha, alpha, st);
 }
 
 template <int R, int OP, int CIN, int TZ, int TY, int YPT, int PREF>
-int launch_stream3d(const float* in, float* out, const Geo& G, const Weights& Wt, float alpha, int mode,
-                    cudaStream_t st) {
-  const int map = pick_map<CIN>(G, R);
-  if (mode == PDE_MODE_FAST) {
-    if (map == MAP_PAIRS)
-      return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_PAIRS, MODE_FAST>(in, out, G, Wt, alpha, alpha, st);
-    if (map == MAP_ROWS_PP0)
-      return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_ROWS_PP0, MODE_FAST>(in, out, G, Wt, alpha, alpha, st);
-    return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_ROWS_GEN, MODE_FAST>(in, out, G, Wt, alpha, alpha, st);
-  }
-  if (map == MAP_PAIRS)
-    return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_PAIRS, MODE_EXACT>(in, out, G, Wt, alpha, alpha, st);
-  if (map == MAP_ROWS_PP0)
-    return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_ROWS_PP0, MODE_EXACT>(in, out, G, Wt, alpha, alpha, st);
-  return launch_stream3d_k<R, OP, CIN, TZ, TY, YPT, PREF, MAP_ROWS_GEN, MODE_EXACT>(in, out, G, Wt, alpha, alpha, st);
+int launch_quads(const float* in, float* out, const Geo& G, const Weights& Wt, float alpha, int mode, int map,
+                 cudaStream_t st) {
+  if (map == MAP_QUADS_PP0)
+    return launch_stream3d<R, OP, CIN, TZ, TY, YPT, PREF, MAP_QUADS_PP0>(in, out, G, Wt, alpha, mode, st);
+  return launch_stream3d<R, OP, CIN, TZ, TY, YPT, PREF, MAP_QUADS_GEN>(in, out, G, Wt, alpha, mode, st);
 }
 
 // Tile configurations of the streaming kernels.  Candidate 0 is the default
@@ -233,10 +236,24 @@ int launch_candidate(int cand, const float* in, float* out, const Geo& G, const 
 template <int R, int OP, int CIN, int TZ, int TY, int YPT, int PREF>
 int launch_selected(int kind, const float* in, float* out, const Geo& G, const Weights& W, float alpha, int mode,
                     cudaStream_t st) {
-  const int cand = g_s3_sel[kind][R - 1];
-  if (cand > 0 && mode == PDE_MODE_EXACT && pick_map<CIN>(G, R) == MAP_PAIRS)
-    return launch_candidate<R, OP, CIN>(cand, in, out, G, W, alpha, st);
-  return launch_stream3d<R, OP, CIN, TZ, TY, YPT, PREF>(in, out, G, W, alpha, mode, st);
+  const int cand = g_s3_sel[kind][R - 1], map = pick_map<CIN>(G, R);
+  if (map == MAP_PAIRS) {
+    if (cand > 0 && mode == PDE_MODE_EXACT) return launch_candidate<R, OP, CIN>(cand, in, out, G, W, alpha, st);
+    return launch_stream3d<R, OP, CIN, TZ, TY, YPT, PREF, MAP_PAIRS>(in, out, G, W, alpha, mode, st);
+  }
+  if constexpr (OP == OP_GRAD) {
+    // A Grad on quad rows spends its time on the cells of its z tiles, the padding
+    // included: the tile width with fewer (301 x 255 x 189, order 2 / 4: 128 wide 60 / 73
+    // us, the alternative 56 / 60 us; 127 x 333 x 451, no less padding: 65 / 81 against
+    // 75 / 93).
+    constexpr int ALT = R == 1 ? 64 : 192;
+    auto padded = [&](int tz) { return (G.ext[2] + tz - 1) / tz * tz; };
+    if (padded(ALT) < padded(128))
+      return launch_quads<R, OP, 1, ALT, R == 1 ? 16 : 8, 4, 4>(in, out, G, W, alpha, mode, map, st);
+    return launch_quads<R, OP, 1, 128, 8, R == 1 ? 8 : 4, 4>(in, out, G, W, alpha, mode, map, st);
+  } else {
+    return launch_quads<R, OP, CIN, TZ, TY, YPT, PREF>(in, out, G, W, alpha, mode, map, st);
+  }
 }
 
 // The flat 1D TMA view addresses floats with int32 coordinates, including rows
@@ -602,22 +619,22 @@ Fill3 fill_table(const PdeBCRules& R) {
 }
 
 // One step of the streaming rollout.  Tiles by plane addressing (pick_map): the
-// double-row map's, or the row maps' (one copy per row) for odd sides.
+// double-row map's, or the quad-row maps' for odd sides.
 int launch_heat_stream(const float* src, float* dst, const Geo& G, const Weights& W, float alpha, float dt,
                        cudaStream_t st) {
   const int map = pick_map<1>(G, G.order / 2);
   if (G.order == 2) {
     if (map == MAP_PAIRS)
       return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
-    if (map == MAP_ROWS_PP0)
-      return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_ROWS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
-    return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_ROWS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+    if (map == MAP_QUADS_PP0)
+      return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_QUADS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+    return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_QUADS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
   }
   if (map == MAP_PAIRS)
     return launch_stream3d_k<2, OP_HEAT, 1, 128, 16, 4, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
-  if (map == MAP_ROWS_PP0)
-    return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_ROWS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
-  return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_ROWS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+  if (map == MAP_QUADS_PP0)
+    return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_QUADS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
+  return launch_stream3d_k<2, OP_HEAT, 1, 64, 32, 8, 4, MAP_QUADS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
 }
 
 // The one-step streaming 3D rollout: per step the fill of the source's boundary in

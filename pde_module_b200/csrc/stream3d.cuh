@@ -3,9 +3,9 @@
 // A block owns a (TY x TZ) tile of interior (y, z) columns and marches along
 // X (the slowest axis) over a chunk of planes.  One producer warp brings each
 // input plane of the tile (TY + 2R rows of TZ + 2R cells plus an alignment
-// lead) into a ring of S shared-memory stages with 1D TMA bulk-tensor copies,
-// one per row: the array's row pitch is arbitrary (e.g. 514 floats), so a 3D
-// tensor map's 16-byte stride rule cannot be met.  Each stage has a "full"
+// lead) into a ring of S shared-memory stages with TMA copies of every second or
+// fourth row: the array's row pitch is arbitrary (e.g. 514 floats), so a map of
+// single rows cannot meet the 16-byte stride rule.  Each stage has a "full"
 // mbarrier (TMA bytes landed) and an "empty" mbarrier (every consumer warp is
 // done with the plane); there is no block-wide barrier in the plane loop.
 //
@@ -38,26 +38,32 @@ struct S3Params {
   float alpha;
   float dt;             // OP_HEAT: the Euler step
   float* out;
+  const float* in;      // quad rows: the array, its floats and the rows of its whole quadruples
+  int total, full_rows;
   uint64_t wait_ns;     // bound of every mbarrier wait
   float negzero;        // -0.0f: the addend of the packed products (not a compile-time constant)
 };
 
 __host__ __device__ constexpr int round4(int v) { return (v + 3) & ~3; }
 
-// Plane addressing: MAP_ROWS_GEN / MAP_ROWS_PP0 bring each tile row with its
-// own 1D TMA copy (the lead of a row inside its 16-byte aligned copy varies
-// with the plane in the GEN case, is fixed in the PP0 case); MAP_PAIRS views
-// the array as (2*Z*CIN, Y/2, X) "double rows" (pitch 8*Z*CIN bytes, a
-// multiple of 16 when Z is even), so a plane tile arrives as two 2D boxes:
-// the even rows and the odd rows.
-enum { MAP_ROWS_GEN = 0, MAP_ROWS_PP0 = 1, MAP_PAIRS = 2 };
+// Plane addressing.  MAP_PAIRS views the array as (2*Z*CIN, Y/2, X) "double rows"
+// (pitch 8*Z*CIN bytes, a multiple of 16 when Z is even), so a plane tile arrives as
+// two boxes: the even rows and the odd rows.  The quad-row maps take every other
+// shape: four rows on are 16*Z*CIN bytes, a multiple of 16 for any Z, so the array is
+// (4*Z*CIN, X*Y/4) "quadruple rows" and a plane tile four boxes, one per row class
+// (flat row mod 4).  (One copy per row kept the copy unit busy with requests: 301 x 255
+// x 189 Grad of order 4 took 88 us, the wider tiles less than the narrow ones.)  The
+// lead of a row inside its 16-byte aligned copy varies with the plane in the GEN case and
+// is fixed in the PP0 case.  The map holds whole quadruples; a tile that reaches the
+// array's last X*Y mod 4 rows copies its plane row by row.
+enum { MAP_QUADS_GEN = 0, MAP_QUADS_PP0 = 1, MAP_PAIRS = 2 };
 
 // Arithmetic of one output row: MODE_EXACT follows the reference sum term by
 // term (every product and sum rounded separately); MODE_FAST sums the taps
 // that share a weight first and uses FMA with alpha folded into the weights.
 enum { MODE_EXACT = 0, MODE_FAST = 1 };
 
-template <int R, int OP, int CIN, int TZ, int TY, int YPT, int PREF, int MAPK = MAP_ROWS_PP0, int MODE = MODE_EXACT>
+template <int R, int OP, int CIN, int TZ, int TY, int YPT, int PREF, int MAPK = MAP_QUADS_PP0, int MODE = MODE_EXACT>
 struct S3Cfg {
   // z pairs (scalar Laplacian or Grad, radius 2, double-row map, exact): a
   // consumer lane owns two adjacent z cells, an 8-byte aligned pair in every
@@ -72,11 +78,13 @@ struct S3Cfg {
   static constexpr int THREADS = NCONS + 32;                     // + one producer warp
   static constexpr int ROWS = TY + 2 * R;
   static constexpr int W = round4(3 + (TZ + 2 * R) * CIN);  // TMA box (floats)
-  static constexpr int WP = (W + 31) & ~31;                 // smem row pitch: 128-byte aligned rows
   static constexpr int S = R + 1 + PREF;                    // stages: centre .. newest + prefetch
   // MAP_PAIRS: each half (even / odd rows) is a dense [ROWS/2][W] box, 128-byte aligned
   static constexpr int HALF = ((ROWS / 2) * W + 31) & ~31;
-  static constexpr int STAGE_FLOATS = (MAPK == MAP_PAIRS) ? 2 * HALF : ROWS * WP;
+  // quad rows: window row m is row m / 4 of box m % 4
+  static constexpr int QROWS = (ROWS + 3) / 4;
+  static constexpr int QUART = (QROWS * W + 31) & ~31;
+  static constexpr int STAGE_FLOATS = (MAPK == MAP_PAIRS) ? 2 * HALF : 4 * QUART;
   // Grad: the tile's TY output rows of a plane (3 TZ floats each, placed at the
   // row's offset within a 128-byte line: pitch 3 TZ + 32); two planes' buffers
   // where two blocks per SM still fit, else one (and a second barrier per plane)
@@ -350,8 +358,8 @@ __global__ void __launch_bounds__(S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MOD
                                    (S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MODE>::THREADS > 320 ? 1 : 2))
     stream3d_kernel(const __grid_constant__ CUtensorMap tmap, const S3Params P, const FastW FW) {
   using C = S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MODE>;
-  constexpr bool PP0 = (MAPK != MAP_ROWS_GEN);
-  constexpr int ROWS = C::ROWS, W = C::W, WP = C::WP, S = C::S, T = 2 * R + 1;
+  constexpr bool PP0 = (MAPK != MAP_QUADS_GEN);
+  constexpr int ROWS = C::ROWS, W = C::W, S = C::S, T = 2 * R + 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* smem = reinterpret_cast<float*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * C::STAGE_FLOATS);
@@ -394,16 +402,38 @@ __global__ void __launch_bounds__(S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MOD
           dead = true;
           flag_error(PDE_ERR_TIMEOUT);
         }
-        if (wl == 0) mbar_arrive_expect_tx(&full[s], ROWS * W * 4);
-        __syncwarp();
         if constexpr (MAPK == MAP_PAIRS) {
+          if (wl == 0) mbar_arrive_expect_tx(&full[s], ROWS * W * 4);
+          __syncwarp();
           // even rows (p = 0) and odd rows (p = 1) of the tile: (y0 - R) is even
           if (wl < 2)
             tma_load_3d(smem + s * C::STAGE_FLOATS + wl * C::HALF, &tmap, (wl * row_f + (z0 - R) * CIN) & ~3,
                         (y0 - R) >> 1, xs - R + i, &full[s]);
         } else {
-          for (int r = wl; r < ROWS; r += 32)
-            tma_load_1d(smem + (s * ROWS + r) * WP, &tmap, (rowf + r * row_f) & ~3, &full[s]);
+          float* st = smem + s * C::STAGE_FLOATS;
+          const int fr = (xs - R + i) * P.Y + (y0 - R);  // flat row of tile row 0
+          if (fr + ROWS <= P.full_rows) {
+            if (wl == 0) mbar_arrive_expect_tx(&full[s], 4 * C::QROWS * W * 4);
+            __syncwarp();
+            if (wl < 4)
+              tma_load_3d(st + wl * C::QUART, &tmap, (((fr + wl) & 3) * row_f + (z0 - R) * CIN) & ~3, (fr + wl) >> 2, 0,
+                          &full[s]);
+          } else {  // rows past the map's whole quadruples: whole 16-byte units of the array, row by row
+            auto row_bytes = [&](int r) {
+              if (r >= ROWS) return 0;
+              const int n = (P.total - ((rowf + r * row_f) & ~3)) & ~3;
+              return 4 * (n < 0 ? 0 : n > W ? W : n);
+            };
+            int bytes = row_bytes(wl) + row_bytes(wl + 32);
+            bytes = __reduce_add_sync(0xffffffffu, bytes);
+            if (wl == 0) mbar_arrive_expect_tx(&full[s], (uint32_t)bytes);
+            __syncwarp();
+            for (int r = wl; r < ROWS; r += 32) {
+              const int nb = row_bytes(r);
+              if (nb > 0)
+                bulk_load(st + (r & 3) * C::QUART + (r >> 2) * W, P.in + ((rowf + r * row_f) & ~3), (uint32_t)nb, &full[s]);
+            }
+          }
         }
         rowf += plane_f;
         ++issued;
@@ -427,13 +457,13 @@ __global__ void __launch_bounds__(S3Cfg<R, OP, CIN, TZ, TY, YPT, PREF, MAPK, MOD
     constexpr int M = YPT + 2 * R;                // centre-plane rows a thread reads
     const int row0 = yg * YPT;                    // first stage row of the thread's window
     // offset (floats) of window row m (stage row row0 + m) inside a stage, without its lead;
-    // MAP_PAIRS: row0 is even (YPT even), so row0 + m has the parity of m
-    static_assert(MAPK != MAP_PAIRS || (YPT % 2 == 0), "pairs need an even row count per thread");
+    // MAP_PAIRS: row0 is even (YPT even), so row0 + m has the parity of m; quad rows: a multiple of 4
+    static_assert(YPT % (MAPK == MAP_PAIRS ? 2 : 4) == 0, "a thread's window starts at a row class of the tile");
     auto rowoff = [&](int m) -> int {
       if constexpr (MAPK == MAP_PAIRS) return (m & 1) * C::HALF + (m >> 1) * W;
-      else return m * WP;
+      else return (m & 3) * C::QUART + (m >> 2) * W;
     };
-    const float* smem_c = smem + ((MAPK == MAP_PAIRS) ? (row0 >> 1) * W : row0 * WP) + cofs;
+    const float* smem_c = smem + (row0 >> (MAPK == MAP_PAIRS ? 1 : 2)) * W + cofs;
 
     float w[T];
 #pragma unroll

@@ -65,27 +65,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// 1D tiled TMA load of one box into shared memory, completion counted in bytes
-// on the mbarrier.  The coordinate must be a multiple of 4 floats (16 bytes).
-__device__ __forceinline__ void tma_load_1d(void* dst, const CUtensorMap* map, int32_t c0, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.1d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// 2D tiled TMA load (coordinate c0 innermost, must be a multiple of 16 bytes).
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int32_t c0, int32_t c1,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// 3D tiled TMA load (c0 innermost, a multiple of 16 bytes).
+// 3D tiled TMA load of one box into shared memory, completion counted in bytes on the
+// mbarrier (coordinate c0 innermost, a multiple of 16 bytes).
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2,
                                             uint64_t* bar) {
   asm volatile(
@@ -93,6 +74,14 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       "[%5];" ::"r"(smem_u32(dst)),
       "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
       : "memory");
+}
+
+// Untiled bulk load of whole 16-byte units, completion counted on the mbarrier.
+__device__ __forceinline__ void bulk_load(float* sdst, const float* gsrc, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(sdst)),
+               "l"((uint64_t)__cvta_generic_to_global(gsrc)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 // Bulk store shared -> global (no tensor map): both addresses 16-byte aligned,
@@ -127,36 +116,6 @@ inline EncodeTiledFn get_encode_fn() {
       fn = (EncodeTiledFn)p;
   }
   return fn;
-}
-
-// Flat 1D fp32 view of `count` floats, box of `box` floats (multiple of 4, <= 256).
-inline bool encode_1d(CUtensorMap* m, const float* base, uint64_t count, uint32_t box) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[1] = {count};
-  cuuint64_t strides[1] = {4};  // unused for rank 1
-  cuuint32_t boxd[1] = {box};
-  cuuint32_t es[1] = {1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 1, (void*)base, dims, strides, boxd, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
-// 2D fp32 view: inner extent n0 floats with row pitch pitch0 floats (pitch0*4
-// multiple of 16), n1 rows; box (b0, b1).
-inline bool encode_2d(CUtensorMap* m, const float* base, uint64_t n0, uint64_t n1, uint64_t pitch0, uint32_t b0,
-                      uint32_t b1) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {n0, n1};
-  cuuint64_t strides[1] = {pitch0 * 4};
-  cuuint32_t boxd[2] = {b0, b1};
-  cuuint32_t es[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)base, dims, strides, boxd, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
 }
 
 // 3D fp32 view (n0 innermost) with byte strides s1, s2 (multiples of 16); box (b0, b1, 1).

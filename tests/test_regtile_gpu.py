@@ -205,3 +205,25 @@ def test_weakly_compressible_tile_rule(shape):
     ref_m, ref_r = acm.wc_rk2(m, rho, ug, rg, dx, 1, nu, eps, c2, rho0, dt, 2)
     assert np.array_equal(got_m.cpu().numpy(), ref_m)
     assert np.array_equal(got_r.cpu().numpy(), ref_r)
+
+
+# X*Y mod 4 = 1, 2, 3 and 0; rows of every length mod 4; tiles of one and of several
+# row quadruples; z of one, two and three tiles
+@pytest.mark.parametrize("shape", [(9, 9, 9), (7, 10, 11), (9, 11, 70), (11, 12, 67), (6, 35, 133), (10, 41, 187),
+                                   (5, 130, 261)])
+@pytest.mark.parametrize("order,extra", [(2, 0), (4, 0), (2, 1)])
+def test_streaming_quad_rows(shape, order, extra):
+    """The 3D operators on shapes whose rows arrive four apart, up to the array's last
+    X*Y mod 4 rows."""
+    g = order // 2 + extra
+    rng = np.random.default_rng(shape[2] + order)
+    u = rng.standard_normal(shape + (3,)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    s = u[..., :1]
+    for n in (1, 3):
+        got = P.Laplacian(n, 0.3, g, order=order)(dev(u[..., :n]), 0.7).cpu().numpy()
+        assert np.array_equal(got, fdm.laplacian(u[..., :n], 0.3, g, 0.7, order)), n
+    got = P.Grad(1, shape + (1,), 0.3, g, order=order)(dev(s), 0.7).cpu().numpy()
+    assert np.array_equal(got, fdm.grad(s, 0.3, g, 0.7, order).reshape(got.shape))
+    got = P.Divergence(3, shape + (3,), 0.3, g, order=order)(dev(u), 0.7).cpu().numpy()
+    assert np.array_equal(got, fdm.divergence(u, 0.3, g, 0.7, order).reshape(got.shape))
