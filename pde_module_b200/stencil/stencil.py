@@ -23,6 +23,9 @@ def tuplify(x: Any) -> tuple:
     return (x,)
 
 
+_REGISTRY = {phase: f"_{phase}_list" for phase in ("setup", "before_forward", "after_forward")}
+
+
 class Stencil:
     initial: bool = True
     device: Optional[torch.device] = None
@@ -47,7 +50,7 @@ class Stencil:
         raise NotImplementedError("forward method in Stencil Object must be implemented by the user")
 
     def _registry(self, phase: str) -> list:
-        name = f"_{phase}_list"
+        name = _REGISTRY[phase]
         reg = self.__dict__.get(name)
         if reg is None:
             found = []
