@@ -232,14 +232,14 @@ int pde_bc_compile(const PdeBCGroup* groups, int32_t ngroups, const PdeGrid* gri
  * when the Laplacian output's ghost cells are zero).
  * u_in: initial field; u_out: result; work: scratch of the same size (used as the
  * ping-pong buffer when nsteps > steps_per_pass).  u_out may equal u_in.
- * steps_per_pass: temporal-blocking depth k (0 = choose).  2D (Z == 1) grids use
- * shared-memory tiles with k steps per pass.  3D grids whose interior has at
- * least 3 cells per axis stream along X with k steps per pass (k at most 4 for
- * one component, 2 for more; deeper requests run at that depth).  At k = 1 a
- * scalar field whose shape takes the double-row map (even Y and Z, plane pitch
- * a multiple of 4 floats, even g - R) runs a surface fill and the TMA streaming
- * heat step per step, and 0 chooses k = 1 there; otherwise 0 chooses 2 for
- * order 2 and 1 for order 4 (pde_heat_pass_depth).  Smaller 3D grids take one
+ * steps_per_pass: temporal-blocking depth k (0 = choose).  2D (Z == 1) scalar
+ * grids with every face filled hold their windows in registers, k steps per pass
+ * (chosen by a cost model); other 2D grids use shared-memory tiles (0 = 8).  3D
+ * scalar fields with at least 3 interior cells per axis and 16-byte aligned buffers
+ * run, at 0 or 1, a surface fill and the TMA streaming heat step per step; deeper
+ * requests, and fields of several components, stream along X with k steps per pass
+ * (at most 4 for one component, 2 for more; deeper requests run at that depth;
+ * 0 = 2 for order 2, 1 for order 4).  Smaller 3D grids take one
  * step per pass.  The input is never written (the streaming path copies it once
  * into a buffer of the call unless u_out == u_in).
  * Constant-valued groups only: rules with a ramp group (has_ramp) give
@@ -272,8 +272,10 @@ int pde_heat_rollout_from(const float* u_in, float* u_out, float* work, const Pd
                           int32_t nsteps, int32_t steps_per_pass, double t0, double t_step,
                           int32_t n0, void* stream);
 
-/* Steps per pass pde_heat_rollout uses on this grid for a steps_per_pass
- * request (0 = choose), or a negative status.  Needs no GPU. */
+/* Steps per pass of the shared-memory and blocked kernels on this grid for a
+ * steps_per_pass request (0 = choose; the depth that slabs of the grid take), or a
+ * negative status.  pde_heat_rollout itself, left to choose, may run another depth on
+ * its register and streaming paths.  Needs no GPU. */
 int pde_heat_pass_depth(const PdeGrid* grid, int32_t ncomp, int32_t steps_per_pass);
 
 /* ---- differentiable heat rollout (new: the reference has the forward loop
@@ -399,7 +401,7 @@ int pde_ldc_slab_step(int32_t phase, float* u, float* u_star, const float* p_in,
  * (out_prev, out_cur) = (u^{n0+nsteps-1}, u^{n0+nsteps}); src_cell < 0: no source.
  * lstates (NULL or nsteps fields): lstates[j] = L(u^{n0+j}) on the cells inside
  * the node ring, 0 elsewhere (the Laplacian each step forms).  work: 2 fields.
- * steps_per_pass: temporal-blocking depth (0 = 8). */
+ * steps_per_pass: temporal-blocking depth (0 = chosen by a cost model). */
 int pde_wave_forward(const float* K, const float* u_prev, const float* u_cur, float* out_prev, float* out_cur,
                      const float* src, int64_t src_cell, int32_t n0, int32_t nsteps, int32_t steps_per_pass,
                      float* lstates, float* work, const PdeGrid* grid, void* stream);
@@ -417,8 +419,8 @@ int pde_wave_adjoint(const float* K, const float* mu_next, const float* mu_next2
  * paired launches: each launch advances every tile through up to
  * steps_per_pass steps of both, so the two interleave on each SM.  Results are
  * bit-identical to the two calls made separately.  Either step count may be 0
- * (that part's pointers may then be NULL).  The pass depth is steps_per_pass or
- * the deepest below it whose shared-memory region fits.  work: 6 fields. */
+ * (that part's pointers may then be NULL).  The pass depth is steps_per_pass (0:
+ * chosen by a cost model) or the deepest below it whose window fits.  work: 6 fields. */
 int pde_wave_pair(const float* K, const float* u_prev, const float* u_cur, int32_t n0, int32_t nsteps_fwd,
                   float* lstates_fwd, const float* mu_next, const float* mu_next2, float* mu_out, float* mu_out_next,
                   const float* lstates_adj, float* grad_K, int32_t nsteps_adj, const float* src, int64_t src_cell,

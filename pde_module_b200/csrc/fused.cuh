@@ -75,15 +75,6 @@ __device__ __forceinline__ float bc_eval(const Geo& G, const PdeBCRules& Rl, con
   return U(c0, c1, c2, v);
 }
 
-// u2 at a cell of a 2D grid: cells strictly inside the node ring are neither
-// boundary nodes nor ghosts, so their boundary-filled value is the input value.
-template <class Acc>
-__device__ __forceinline__ float bc_eval2d(const Geo& G, const PdeBCRules& Rl, const Acc& U, int64_t i, int64_t j,
-                                           int v) {
-  if (i > G.g && i < G.n[0] - 1 - G.g && j > G.g && j < G.n[1] - 1 - G.g) return U(i, j, 0, v);
-  return bc_eval(G, Rl, U, i, j, 0, v);
-}
-
 struct GlobalAcc {
   const float* u;
   int64_t s0, s1;  // cell strides

@@ -381,7 +381,7 @@ int pde_grad_ex(const float* in, float* out, const PdeGrid* grid, int32_t ncomp,
   const Weights W = d1_weights(G.order, grid->dx);
   cudaStream_t st = as_stream(stream);
   if (ncomp == 1 && stream3d_ok(in, G, 1)) {
-    // default tile (fast mode, and shapes without the double-row map): 128 x 8, 4 rows per thread
+    // default tile (fast mode and candidate 0 on the double-row map): 128 x 8, 4 rows per thread
     if (G.order == 2) return launch_selected<1, OP_GRAD, 1, 128, 8, 4, 4>(S3K_GRAD, in, out, G, W, alpha, mode, st);
     return launch_selected<2, OP_GRAD, 1, 128, 8, 4, 4>(S3K_GRAD, in, out, G, W, alpha, mode, st);
   }
@@ -730,7 +730,7 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
   int k = heat_depth(G, ncomp, steps_per_pass);
   if (k > nsteps) k = nsteps;
   // a depth left open streams one step per pass on any shape (odd sides too, where the
-  // row maps take 47 us a step on 255 x 191 x 319 against 163 of the blocked kernel)
+  // quad-row map takes 43 us a step on 255 x 191 x 319 against 163 of the blocked kernel)
   if (s3d && (steps_per_pass == 0 || k == 1) && heat_stream_shape(G, ncomp) && aligned16(u_in) && aligned16(u_out) && aligned16(work))
     return heat3d_split_run(u_in, u_out, work, G, W, rules, alpha, dt, nsteps, t0, tstep, n0, input_scratch, st);
   const int npasses = (nsteps + k - 1) / k;

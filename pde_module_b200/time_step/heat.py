@@ -4,8 +4,8 @@ Runs ``nsteps`` of the reference's explicit step (examples/2D_Heat_Equation.py:5
 
     u2 = BC(u);  lap = Laplacian(u2, alpha);  u = ForwardEuler(u2, lap, dt)
 
-in fused sm_100a kernels: 2D grids advance k steps per pass out of shared-memory
-tiles (temporal blocking), 3D grids one fused step per pass.  The result is
+in fused sm_100a kernels: 2D grids advance k steps per pass on windows held in
+registers or shared memory (temporal blocking), 3D grids one fused step per pass.  The result is
 bit-identical to running the three modules of this package step by step (the
 Laplacian module's ghost cells are zero, so Euler copies the boundary-filled
 ghosts through).
