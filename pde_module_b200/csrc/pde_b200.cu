@@ -243,13 +243,13 @@ int launch_selected(int kind, const float* in, float* out, const Geo& G, const W
   }
   if constexpr (OP == OP_GRAD) {
     // A Grad on quad rows spends its time on the cells of its z tiles, the padding
-    // included: the tile width with fewer (301 x 255 x 189, order 2 / 4: 128 wide 60 / 73
-    // us, the alternative 56 / 60 us; 127 x 333 x 451, no less padding: 65 / 81 against
-    // 75 / 93).
-    constexpr int ALT = R == 1 ? 64 : 192;
+    // included: 128 wide, or the alternative where it pads no more (us at 301 x 255 x 189,
+    // order 2 / 4: 60 / 73 and 53 / 54; 255 x 257 x 259, order 2: 73 and 60; 127 x 333 x
+    // 451, order 4, where the alternative pads more: 82 and 87).
+    constexpr int ALT = R == 1 ? 96 : 192;
     auto padded = [&](int tz) { return (G.ext[2] + tz - 1) / tz * tz; };
-    if (padded(ALT) < padded(128))
-      return launch_quads<R, OP, 1, ALT, R == 1 ? 16 : 8, 4, 4>(in, out, G, W, alpha, mode, map, st);
+    if (padded(ALT) <= padded(128))
+      return launch_quads<R, OP, 1, ALT, R == 1 ? 8 : 12, R == 1 ? 8 : 4, 4>(in, out, G, W, alpha, mode, map, st);
     return launch_quads<R, OP, 1, 128, 8, R == 1 ? 8 : 4, 4>(in, out, G, W, alpha, mode, map, st);
   } else {
     return launch_quads<R, OP, CIN, TZ, TY, YPT, PREF>(in, out, G, W, alpha, mode, map, st);

@@ -87,11 +87,12 @@ struct S3Cfg {
   static constexpr int STAGE_FLOATS = (MAPK == MAP_PAIRS) ? 2 * HALF : 4 * QUART;
   // Grad: the tile's TY output rows of a plane (3 TZ floats each, placed at the
   // row's offset within a 128-byte line: pitch 3 TZ + 32); two planes' buffers
-  // where two blocks per SM still fit, else one (and a second barrier per plane)
+  // where the blocks per SM still fit (two up to 320 threads, else one), else one (and a
+  // second barrier per plane: 192 x 12 tiles of 301 x 255 x 189, order 4, 53 against 74 us)
   static constexpr int OROW = 3 * TZ + 32;
   // + 128: the base is rounded up to a 128-byte boundary at run time
   static constexpr size_t SMEM_BASE = (size_t)S * STAGE_FLOATS * 4 + (size_t)2 * S * 8 + 128;
-  static constexpr int OBUFS = (SMEM_BASE + (size_t)2 * TY * OROW * 4 <= 113 * 1024) ? 2 : 1;
+  static constexpr int OBUFS = (SMEM_BASE + (size_t)2 * TY * OROW * 4 <= (THREADS > 320 ? 226 : 113) * 1024) ? 2 : 1;
   static constexpr int OBUF_FLOATS = (OP == OP_GRAD) ? OBUFS * TY * OROW : 0;
   static constexpr size_t SMEM = SMEM_BASE + (size_t)OBUF_FLOATS * 4;
   static_assert(NCONS % 32 == 0, "whole consumer warps");
