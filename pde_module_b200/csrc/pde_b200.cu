@@ -620,18 +620,26 @@ Fill3 fill_table(const PdeBCRules& R) {
 
 // One step of the streaming rollout.  Tiles by plane addressing (pick_map): the
 // double-row map's, or the quad-row maps' for odd sides: the fastest of a sweep over
-// sides of 64 to 320.  On the double-row map narrow tiles pad less (us per step, 256 x
-// 192 x 320, order 2: 37.5, 128 wide 40.8; 300^3, order 4: 67.8, 128 wide 74.8).
+// sides of 64 to 320.  On the double-row map narrow tiles pad less and leave more blocks
+// to balance, wide ones read fewer halo cells, which counts once the fields are far
+// beyond L2 (us per step, 64 / 128 wide, order 2: 256 x 192 x 320 37.5 / 40.8, 320^3 71.0 /
+// 74.6, 384^3 115 / 109, 512^3 319 / 249; order 4: 300^3 67.8 / 74.8, 320^3 78.2 / 85.1,
+// 384^3 121.6 / 120.1, 512^3 310 / 273): the line is drawn between 320^3 and 384^3.
 int launch_heat_stream(const float* src, float* dst, const Geo& G, const Weights& W, float alpha, float dt,
                        cudaStream_t st) {
   const int map = pick_map<1>(G, G.order / 2);
+  const bool wide = G.n[0] * G.n[1] * G.n[2] > (44LL << 20);
   if (G.order == 2) {
+    if (map == MAP_PAIRS && wide)
+      return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
     if (map == MAP_PAIRS)
       return launch_stream3d_k<1, OP_HEAT, 1, 64, 16, 8, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
     if (map == MAP_QUADS_PP0)
       return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_QUADS_PP0, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
     return launch_stream3d_k<1, OP_HEAT, 1, 128, 16, 8, 3, MAP_QUADS_GEN, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
   }
+  if (map == MAP_PAIRS && wide)
+    return launch_stream3d_k<2, OP_HEAT, 1, 128, 16, 4, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
   if (map == MAP_PAIRS)
     return launch_stream3d_k<2, OP_HEAT, 1, 64, 16, 4, 4, MAP_PAIRS, MODE_EXACT>(src, dst, G, W, alpha, alpha, st, dt);
   if (map == MAP_QUADS_PP0)
