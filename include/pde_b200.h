@@ -488,7 +488,10 @@ typedef struct PdeBatchPlan {
   int32_t    register_tiles;  /* windows in registers (else in shared memory)       */
 } PdeBatchPlan;
 
-/* Device bytes `work` must hold for these grids and tile (0 = default). */
+/* Device bytes of `work` for these grids and tile (0 = default): the table and a
+ * progress word per tile, as many as any depth and kind may need.  pde_batch_plan
+ * takes less as long as it holds the words of the shared-memory tiles, and then
+ * runs register tiles only where theirs fit too. */
 int pde_batch_work_bytes(const PdeBatchGrid* grids, int32_t ngrids, int32_t tile_x, int32_t tile_y,
                          uint64_t* bytes);
 /* Validate the grids, choose the launch (tile 0 and steps_per_pass 0: chosen by the

@@ -1683,8 +1683,24 @@ constexpr size_t BATCH_QUEUE_OFF_ALIGN = 256;
 size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // work layout: [descriptor table][queue counter, 256 B][progress: u32 per tile]
-bool batch_layout(const PdeBatchGrid* grids, int ngrids, int tx, int ty, int64_t* total_tiles, size_t* table_bytes,
-                  size_t* bytes) {
+size_t batch_table_bytes(int ngrids) { return round_up((size_t)ngrids * sizeof(BatchGridDev), BATCH_QUEUE_OFF_ALIGN); }
+size_t batch_work_for(int ngrids, int64_t tiles) {
+  return batch_table_bytes(ngrids) + BATCH_QUEUE_OFF_ALIGN + (size_t)tiles * sizeof(unsigned);
+}
+
+// The most register tiles of an axis of n array cells under any depth and ghost
+// width: a given tile covers the box, which is smaller than the array; else
+// rt_grid_tiles takes one or two tiles, or windows of `cap` cells less a halo on
+// both sides that is no wider than the tile left, a third of the window.
+int64_t batch_register_tiles_most(int64_t n, int tile, int cap) {
+  if (tile > 0) return (n + tile - 1) / tile;
+  const int least = cap - 2 * (cap / 3);
+  const int64_t most = (n + least - 1) / least;
+  return most > 2 ? most : 2;
+}
+
+// Shared-memory tiles of tx x ty array cells.
+bool batch_tiles(const PdeBatchGrid* grids, int ngrids, int tx, int ty, int64_t* total_tiles) {
   int64_t tiles = 0;
   for (int i = 0; i < ngrids; ++i) {
     const int64_t X = grids[i].shape[0], Y = grids[i].shape[1];
@@ -1693,8 +1709,6 @@ bool batch_layout(const PdeBatchGrid* grids, int ngrids, int tx, int ty, int64_t
   }
   if (tiles <= 0 || tiles > (1LL << 30)) return false;
   *total_tiles = tiles;
-  *table_bytes = round_up((size_t)ngrids * sizeof(BatchGridDev), BATCH_QUEUE_OFF_ALIGN);
-  *bytes = *table_bytes + BATCH_QUEUE_OFF_ALIGN + (size_t)tiles * sizeof(unsigned);
   return true;
 }
 
@@ -1723,10 +1737,12 @@ int pde_batch_work_bytes(const PdeBatchGrid* grids, int32_t ngrids, int32_t tile
                          uint64_t* bytes) {
   if (!grids || ngrids < 1 || !bytes || tile_x < 0 || tile_y < 0) return PDE_ERR_ARG;
   const int tx = tile_x > 0 ? tile_x : BATCH_TILE_X, ty = tile_y > 0 ? tile_y : BATCH_TILE_Y;
-  int64_t tiles;
-  size_t tb, b;
-  if (!batch_layout(grids, ngrids, tx, ty, &tiles, &tb, &b)) return PDE_ERR_SHAPE;
-  *bytes = b;
+  int64_t tiles, most = 0;
+  if (!batch_tiles(grids, ngrids, tx, ty, &tiles)) return PDE_ERR_SHAPE;
+  for (int i = 0; i < ngrids; ++i)
+    most += batch_register_tiles_most(grids[i].shape[0], tile_x, BRT_ROWS) *
+            batch_register_tiles_most(grids[i].shape[1], tile_y, BRT_COLS);
+  *bytes = batch_work_for(ngrids, most > tiles ? most : tiles);
   return PDE_OK;
 }
 
@@ -1748,23 +1764,27 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
   const int H = batch_halo(kind, order, k);
   if (H > tx || H > ty || tx > 4096 || ty > 4096) return PDE_ERR_ARG;
   int64_t tiles;
-  size_t table_bytes, bytes;
-  if (!batch_layout(grids, ngrids, tx, ty, &tiles, &table_bytes, &bytes)) return PDE_ERR_SHAPE;
-  if (work_bytes < bytes) return PDE_ERR_TOO_LARGE;
+  if (!batch_tiles(grids, ngrids, tx, ty, &tiles)) return PDE_ERR_SHAPE;
+  if (work_bytes < batch_work_for(ngrids, tiles)) return PDE_ERR_TOO_LARGE;
   const int nbuf = kind == PDE_BATCH_HEAT ? 2 : 3;
   const size_t smem = (size_t)nbuf * (tx + 2 * H) * (ty + 2 * H) * sizeof(float);
   if (smem > 227 * 1024) return PDE_ERR_TOO_LARGE;
-  BatchGridDev* host = new BatchGridDev[ngrids];
-  // Register tiles where every grid of the batch takes them: order 2, every face
-  // filled (heat), boxes of two strips and two lanes at least, a given tile that fits.
+  BatchGridDev* host = new BatchGridDev[ngrids]();
+  // Register tiles where every grid of the batch takes them (order 2, every face
+  // filled (heat), boxes of two strips and two lanes at least, a given tile that fits)
+  // and `work` holds a progress word for each.
   const int box_pad = kind == PDE_BATCH_HEAT ? ghost_cells : ghost_cells + 1;
   const int kr = steps_per_pass > 0 ? steps_per_pass : BRT_K;
   bool rt = order == 2 && g_dispatch != PDE_DISPATCH_GENERIC && (kind == PDE_BATCH_WAVE || rt_fills_all_faces(*rules));
+  int64_t rt_tiles = 0;
   for (int i = 0; i < ngrids && rt; ++i) {
     const int64_t BX = grids[i].shape[0] - 2 * box_pad, BY = grids[i].shape[1] - 2 * box_pad;
+    RTGeom& Wi = host[i].W;
     rt = BX >= 8 && BY >= 8 && BX * BY < (1LL << 30) &&
-         rt_grid_tiles((int)BX, (int)BY, kr, BRT_C, BRT_RPT, BRT_ROWS, BRT_COLS, tile_x, tile_y, &host[i].W);
+         rt_grid_tiles((int)BX, (int)BY, kr, BRT_C, BRT_RPT, BRT_ROWS, BRT_COLS, tile_x, tile_y, &Wi);
+    if (rt) rt_tiles += (int64_t)((Wi.BX + Wi.TBX - 1) / Wi.TBX) * Wi.tiles_y;
   }
+  rt = rt && rt_tiles <= (1LL << 30) && work_bytes >= batch_work_for(ngrids, rt_tiles);
   int64_t base = 0;
   int most_x = 0, most_y = 0;
   for (int i = 0; i < ngrids; ++i) {
@@ -1804,6 +1824,20 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
     const Weights W = lap_weights(order, B.dx);
     for (int t = 0; t < 5; ++t) D.w[t] = W.w[t];
   }
+  // the plan, all of it but the block count, before the first call to the device
+  memset(plan, 0, sizeof(*plan));
+  plan->table = work;
+  plan->kind = kind;
+  plan->ngrids = ngrids;
+  plan->total_tiles = (int32_t)base;
+  plan->ghost_cells = ghost_cells;
+  plan->order = order;
+  plan->tile_x = rt ? most_x : tx;
+  plan->tile_y = rt ? most_y : ty;
+  plan->steps_per_pass = rt ? kr : k;
+  plan->register_tiles = rt ? 1 : 0;
+  plan->smem_bytes = (int32_t)smem;
+  if (kind == PDE_BATCH_HEAT) plan->rules = *rules;
   cudaStream_t st = as_stream(stream);
   const cudaError_t ce = cudaMemcpyAsync(work, host, (size_t)ngrids * sizeof(BatchGridDev), cudaMemcpyHostToDevice, st);
   delete[] host;
@@ -1816,20 +1850,7 @@ int pde_batch_plan(int32_t kind, const PdeBatchGrid* grids, int32_t ngrids, int3
   else
     rc = batch_occupancy<BATCH_WAVE, 1>((int)smem, &occ);
   if (rc) return rc;
-  memset(plan, 0, sizeof(*plan));
-  plan->table = work;
-  plan->kind = kind;
-  plan->ngrids = ngrids;
-  plan->total_tiles = rt ? (int32_t)base : (int32_t)tiles;
-  plan->ghost_cells = ghost_cells;
-  plan->order = order;
-  plan->tile_x = rt ? most_x : tx;
-  plan->tile_y = rt ? most_y : ty;
-  plan->steps_per_pass = rt ? kr : k;
-  plan->register_tiles = rt ? 1 : 0;
   plan->blocks = occ * sm_count();
-  plan->smem_bytes = (int32_t)smem;
-  if (kind == PDE_BATCH_HEAT) plan->rules = *rules;
   return PDE_OK;
 }
 
@@ -1854,7 +1875,7 @@ int batch_rollout_run(const PdeBatchPlan* plan, int32_t nsteps, double t0, void*
   ntb += ntb & 1;  // even: the last block writes the parity-0 buffers (the caller's fields)
   if ((int64_t)ntb * plan->total_tiles >= (1LL << 31) - (int64_t)plan->blocks) return PDE_ERR_TOO_LARGE;
   const int kmax = (nsteps + ntb - 1) / ntb;
-  size_t table_bytes = round_up((size_t)plan->ngrids * sizeof(BatchGridDev), BATCH_QUEUE_OFF_ALIGN);
+  const size_t table_bytes = batch_table_bytes(plan->ngrids);
   char* base = static_cast<char*>(plan->table);
   BatchParams P;
   P.grids = reinterpret_cast<const BatchGridDev*>(base);

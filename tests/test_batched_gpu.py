@@ -127,3 +127,40 @@ def test_batched_zero_steps_is_identity():
     P.BatchedHeatRollout(a, dx, alpha, dts)(0)
     for x, f in zip(a, fields):
         assert np.array_equal(x.cpu().numpy(), f)
+
+
+@pytest.mark.parametrize("kind", ["heat", "wave"])
+def test_batched_thin_grids_stay_in_their_work_buffer(kind):
+    """Narrow boxes take more register tiles than shared-memory tiles: the words behind
+    a work buffer of the size asked for stay as they are, and results match the oracle."""
+    boxes = [(150, 50), (300, 61), (661, 25), (25, 25), (28, 57)] * 3
+    pad = 1 if kind == "heat" else 2
+    rng = np.random.default_rng(2)
+    u = []
+    for x, y in boxes:
+        f = np.zeros((x + 2 * pad, y + 2 * pad, 1, 1), dtype=np.float32)
+        f[pad:-pad, pad:-pad, 0, 0] = rng.random((x, y))
+        u.append(f)
+    dev, prev = [torch.from_numpy(f).cuda() for f in u], [torch.from_numpy(f).cuda() for f in u]
+    dx = [1.0 / x for x, _ in boxes]
+    dt = [float(np.float32(0.2 * h * h)) for h in dx]
+    if kind == "heat":
+        roll = P.BatchedHeatRollout(dev, dx, 1.0, dt)
+    else:
+        roll = P.BatchedWaveRollout(dev, prev, dx, dt)
+    need = roll._work.numel()
+    guarded = torch.full((need + 4096,), 0xA5, device="cuda", dtype=torch.uint8)
+    roll._work = guarded[:need]
+    roll.configure()
+    assert roll.plan.register_tiles == 1 and 4 * roll.plan.total_tiles + 256 <= need
+    roll(23)
+    assert P._lib.device_error() == 0
+    assert bool((guarded[need:] == 0xA5).all())
+    for i in range(5):
+        if kind == "heat":
+            spec = fdm.standard_groups(u[i].shape[:3], 1, [("ALL", 1, 0.0, (0,))])
+            assert np.array_equal(dev[i].cpu().numpy(), fdm.heat_rollout(u[i], spec, dx[i], 1, 1.0, dt[i], 23)), boxes[i]
+        else:
+            st = fdm.wave_forward(np.full(u[i].shape, dt[i], np.float32), u[i], None, None, 23, dx[i])
+            assert np.array_equal(dev[i].cpu().numpy()[:, :, 0, 0], st[-1]), boxes[i]
+            assert np.array_equal(prev[i].cpu().numpy()[:, :, 0, 0], st[-2]), boxes[i]
