@@ -64,7 +64,14 @@ struct Reg2 {
   }
 };
 
-// A block's tile and region (tile + halo, within the array and the held rows).
+// A block's tile and region (tile + halo, within the array and the held rows).  A
+// tile's ghosts are filled in its region from the cell two steps inward, so a tile that
+// begins at the high ghosts, or ends at the low ones, takes two cells on that side
+// whatever the halo: at most one more row and one more column than tile and halos.
+__host__ __device__ constexpr int ldc_cap(int halo) {
+  const int most = halo < 2 ? 2 : halo;
+  return (LDC_TX + halo + most) * (LDC_TY + halo + most);
+}
 struct LdcTile {
   int bx0, by0, bx1, by1, rx0, ry0, RX, RY;
   __device__ LdcTile(const LdcRows& D, int halo) {
@@ -72,10 +79,11 @@ struct LdcTile {
     by0 = (int)blockIdx.x * LDC_TY;
     bx1 = min(bx0 + LDC_TX, D.own_hi);
     by1 = min(by0 + LDC_TY, D.Y);
-    rx0 = max(bx0 - halo, D.held_lo);
-    ry0 = max(by0 - halo, 0);
-    RX = min(bx1 + halo, D.held_hi) - rx0;
-    RY = min(by1 + halo, D.Y) - ry0;
+    const int most = max(halo, 2);
+    rx0 = max(bx0 - (bx0 == D.X - D.g ? most : halo), D.held_lo);
+    ry0 = max(by0 - (by0 == D.Y - D.g ? most : halo), 0);
+    RX = min(bx1 + (bx1 == D.g ? most : halo), D.held_hi) - rx0;
+    RY = min(by1 + (by1 == D.g ? most : halo), D.Y) - ry0;
   }
   // fn(region index, x, y) over the region's cells / the tile's cells
   template <class F>
@@ -155,7 +163,7 @@ __global__ void __launch_bounds__(LDC_THREADS) ldc_velocity_kernel(const float* 
                                                                    const PdeBCRules Ru, const LdcConst K) {
   pdl_launch_dependents();
   constexpr int HALO = PREDICT && DIVERGE ? 2 : 1;
-  constexpr int CAP = (LDC_TX + 2 * HALO) * (LDC_TY + 2 * HALO);
+  constexpr int CAP = ldc_cap(HALO);
   __shared__ float2 A[PREDICT ? CAP : 1], B[DIVERGE ? CAP : 1];
   const LdcTile T(D, HALO);
   const H2Params HP = ldc_shape(D);
@@ -218,7 +226,7 @@ __global__ void __launch_bounds__(LDC_THREADS) ldc_project_kernel(const float* _
                                                                    const LdcRows D, const PdeBCRules Ru,
                                                                    const PdeBCRules Rp, const LdcConst K) {
   pdl_launch_dependents();
-  constexpr int CAP = (LDC_TX + 2) * (LDC_TY + 2);
+  constexpr int CAP = ldc_cap(1);
   __shared__ float2 A[CAP];
   __shared__ float Pr[CAP];
   const LdcTile T(D, 1);

@@ -60,3 +60,44 @@ def test_slabs_match_whole_domain(n, slabs, iters, k, steps):
         rows = slice(s.own_lo, s.own_hi)
         assert torch.equal(s.u[s.owned], whole.u[rows]), (s.own_lo, s.own_hi)
         assert torch.equal(s.p[s.owned], whole.p[rows]), (s.own_lo, s.own_hi)
+
+
+@pytest.mark.parametrize("n,g", [(15, 1), (31, 1), (63, 1), (127, 1), (14, 2), (62, 2), (29, 3), (20, 16)])
+def test_ldc_tiles_of_ghosts_alone(n, g):
+    """Velocity tiles (16 rows, 64 columns) that begin at the high ghosts or end at the low
+    ones: a ghost's partner lies two cells inside, beyond the tile's neighbours."""
+    s = P.FractionalStepLDC(n=n, Re=100.0, jacobi_iters=6, dt=1e-3 / n, ghost_cells=g)
+    rng = np.random.default_rng(n)
+    u = (0.1 * rng.standard_normal(tuple(s.u.shape))).astype(np.float32)
+    p = (0.1 * rng.standard_normal(tuple(s.p.shape))).astype(np.float32)
+    s.u.copy_(torch.from_numpy(u))
+    s.p.copy_(torch.from_numpy(p))
+    s.step(2)
+    G = fdm.exterior_groups(u.shape, g)
+    ug = [dict(ids=G["ALL"], type=1, value=0.0, comps=(0, 1)), dict(ids=G["+Y"], type=1, value=1.0, comps=(0,))]
+    pg = [dict(ids=G["ALL"], type=2, value=0.0, comps=(0,))]
+    for _ in range(2):
+        u, p = fdm.ldc_step(u, p, ug, pg, s.dx, g, s.nu, s.dt, 6)
+    assert np.array_equal(s.u.cpu().numpy(), u)
+    assert np.array_equal(s.p.cpu().numpy(), p)
+
+
+@pytest.mark.parametrize("n,cut", [(48, 33), (64, 33), (62, 31)])
+def test_slab_of_one_row_more_than_its_tiles(n, cut):
+    """The last slab owns 17 or 33 rows: its last velocity tile is the ghost row."""
+    from pde_module_b200.time_step.fractional_step import LDCSlab, ldc_slab_steps
+    from pde_module_b200.distributed import exchange_local_slabs
+    X, halo = n + 2, 5
+    whole = P.FractionalStepLDC(n=n, Re=100.0, jacobi_iters=8, jacobi_per_pass=4, dt=1e-3)
+    whole.u.copy_(torch.rand(whole.u.shape, generator=torch.Generator().manual_seed(n)))
+    parts = [LDCSlab(r, n=n, Re=100.0, jacobi_iters=8, jacobi_per_pass=4, dt=1e-3)
+             for r in [(0, cut, 0, cut + halo), (cut, X, cut - halo, X)]]
+    for s in parts:
+        s.u.copy_(whole.u[s.held_lo:s.held_hi])
+    whole.step(2)
+    ldc_slab_steps(parts, 2, lambda fields: exchange_local_slabs(fields, halo))
+    for s in parts:
+        rows = slice(s.own_lo, s.own_hi)
+        assert torch.equal(s.u_star[s.owned], whole._u_star[rows]), (s.own_lo, s.own_hi)
+        assert torch.equal(s.u[s.owned], whole.u[rows]), (s.own_lo, s.own_hi)
+        assert torch.equal(s.p[s.owned], whole.p[rows]), (s.own_lo, s.own_hi)
