@@ -212,6 +212,18 @@ __global__ void __launch_bounds__(BRT_WARPS * 32, 2) batched_rt_kernel(const Bat
         rt_store<C, RPT>(u, (swapped ? out1 : out0) + first, Gd.Y, V);
         rt_store<C, RPT>(um, (swapped ? out0 : out1) + first, Gd.Y, V);
       }
+      // The last block writes the caller's fields: 0 on the ring and the ghosts, which
+      // no window holds, so the tiles at the box's edges may write them at any time.
+      if (tb == P.ntb - 1 && (V.bx0 == 0 || V.by0 == 0 || V.bx1 == W.BX || V.by1 == W.BY)) {
+        const int x0 = V.bx0 + pad, x1 = V.bx1 + pad, y0 = V.by0 + pad, y1 = V.by1 + pad;  // the tile in the array
+        const int ax = V.bx0 == 0 ? 0 : x0, bx = V.bx1 == W.BX ? Gd.X : x1;
+        const int ay = V.by0 == 0 ? 0 : y0, by = V.by1 == W.BY ? Gd.Y : y1;
+        RectWalk wk(by - ay, (int)blockDim.x);
+        for (int i = tid; i < (bx - ax) * (by - ay); i += (int)blockDim.x, wk.next()) {
+          const int x = ax + wk.row, y = ay + wk.col;
+          if (x < x0 || x >= x1 || y < y0 || y >= y1) out0[(size_t)x * Gd.Y + y] = out1[(size_t)x * Gd.Y + y] = 0.0f;
+        }
+      }
     }
     __threadfence();
     __syncthreads();

@@ -164,3 +164,29 @@ def test_batched_thin_grids_stay_in_their_work_buffer(kind):
             st = fdm.wave_forward(np.full(u[i].shape, dt[i], np.float32), u[i], None, None, 23, dx[i])
             assert np.array_equal(dev[i].cpu().numpy()[:, :, 0, 0], st[-1]), boxes[i]
             assert np.array_equal(prev[i].cpu().numpy()[:, :, 0, 0], st[-2]), boxes[i]
+
+
+@pytest.mark.parametrize("rows,tile,k,register", [(24, None, 0, 0), (66, None, 0, 1), (24, None, 4, 1),
+                                                  (24, (64, 64), 8, 0)])
+@pytest.mark.parametrize("nsteps", [1, 2, 23])
+@pytest.mark.parametrize("g", [1, 2])
+def test_batched_wave_zeroes_the_ring(rows, tile, k, register, nsteps, g):
+    """Fields that come in with values on the node ring and the ghosts: those count as 0
+    and are 0 in both levels afterwards, on either kind of tile (22 rows of cells hold no
+    window with a halo of 10)."""
+    shapes = [(70, 90), (131, 40), (rows, 300)]
+    rng = np.random.default_rng(g + nsteps)
+    u = [rng.standard_normal((x + 2 * g, y + 2 * g, 1, 1)).astype(np.float32) for x, y in shapes]
+    now, prev = [torch.from_numpy(f).cuda() for f in u], [torch.from_numpy(f).cuda() for f in u]
+    dx = [1.0 / (x - 1) for x, _ in shapes]
+    K = [float(np.float32(0.2 * h * h)) for h in dx]
+    roll = P.BatchedWaveRollout(now, prev, dx, K, ghost_cells=g, tile=tile, steps_per_pass=k)
+    assert roll.plan.register_tiles == register
+    roll(nsteps)
+    assert P._lib.device_error() == 0
+    for i in range(len(shapes)):
+        f = np.zeros_like(u[i])
+        f[g + 1:-g - 1, g + 1:-g - 1] = u[i][g + 1:-g - 1, g + 1:-g - 1]
+        st = fdm.wave_forward(np.full(f.shape, K[i], np.float32), f, None, None, nsteps, dx[i], ghost=g)
+        assert np.array_equal(now[i].cpu().numpy()[:, :, 0, 0], st[-1]), shapes[i]
+        assert np.array_equal(prev[i].cpu().numpy()[:, :, 0, 0], st[-2]), shapes[i]
