@@ -29,6 +29,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // pdl_wait blocks until the previous kernel has completed and its writes are
 // visible: every global access to data another launch reads or writes comes
 // after it.  Both are no-ops for kernels launched without the attribute.
+// A kernel that waits may be resident while the launch before it still writes what it
+// will read.  It takes its arrays by plain pointers: `const __restrict__` (or __ldg)
+// promises data that is constant for the kernel's whole life, which the compiler may
+// read on a path, or at a point, that the wait does not govern.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) heat_fill3_kernel(float* __restrict__ u, 
 
 // The g outer layers of src into dst (a buffer's first use; the last step's ghosts, as
 // its source had them).
-__global__ void __launch_bounds__(256) heat_copy_shell_kernel(const float* __restrict__ src, float* __restrict__ dst,
+__global__ void __launch_bounds__(256) heat_copy_shell_kernel(const float* src, float* dst,
                                                               Geo G, Shell S) {
   pdl_launch_dependents();
   pdl_wait();
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(1024) heat2d_tb_kernel(const float* __restrict
 // Same arithmetic and order per cell as heat2d_tb_kernel<R, 1, RAMP>; needs
 // RXM x RYM <= MAXC * blockDim.x and < 2^16.
 template <int R, int MAXC, bool RAMP>
-__global__ void __launch_bounds__(1024) heat2d_cells_kernel(const float* __restrict__ in, float* __restrict__ out,
+__global__ void __launch_bounds__(1024) heat2d_cells_kernel(const float* in, float* out,
                                                             const H2Params P, const PdeBCRules Rl) {
   pdl_launch_dependents();  // the next pass may be scheduled; it waits for this one
   extern __shared__ __align__(16) float sm[];

@@ -186,7 +186,7 @@ __device__ __forceinline__ void h3_ztaps(const float* B, int r, float2 cen, floa
 
 template <int R, int K, int N, int TYM, int TZM, int T>
 __global__ void __launch_bounds__(T, (H3Cfg<R, K, N, TYM, TZM, T>::MINB))
-    heat3d_kernel(const float* __restrict__ in, float* __restrict__ out, const H3Params P,
+    heat3d_kernel(const float* in, float* out, const H3Params P,
                   const __grid_constant__ PdeBCRules rules) {
   using Cf = H3Cfg<R, K, N, TYM, TZM, T>;
   constexpr int PP = Cf::P, PS = Cf::PS, PL = Cf::PLANE, C = Cf::C, S = Cf::S, Q = Cf::Q, H = Cf::H, PF = Cf::PF;

@@ -158,8 +158,7 @@ __device__ __forceinline__ float ldc_div_cell(const Get& at, int i, int j, const
 // stays in shared memory for the divergence (a slab runs them one by one: u* rows
 // of the neighbouring slab come between).
 template <bool PREDICT, bool DIVERGE>
-__global__ void __launch_bounds__(LDC_THREADS) ldc_velocity_kernel(const float* __restrict__ u, float* us,
-                                                                   float* __restrict__ rhs, const LdcRows D,
+__global__ void __launch_bounds__(LDC_THREADS) ldc_velocity_kernel(const float* u, float* us, float* rhs, const LdcRows D,
                                                                    const PdeBCRules Ru, const LdcConst K) {
   pdl_launch_dependents();
   constexpr int HALO = PREDICT && DIVERGE ? 2 : 1;
@@ -221,8 +220,7 @@ __device__ __forceinline__ void ldc_project_cell(const GetU& au, const GetP& ap,
   res[1] = add(a1, mul(K.dt, mul(-1.0f, gy)));
 }
 
-__global__ void __launch_bounds__(LDC_THREADS) ldc_project_kernel(const float* __restrict__ us,
-                                                                   const float* __restrict__ p, float* __restrict__ u,
+__global__ void __launch_bounds__(LDC_THREADS) ldc_project_kernel(const float* us, const float* p, float* u,
                                                                    const LdcRows D, const PdeBCRules Ru,
                                                                    const PdeBCRules Rp, const LdcConst K) {
   pdl_launch_dependents();

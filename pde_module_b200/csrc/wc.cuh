@@ -101,8 +101,7 @@ __device__ __forceinline__ float2 wc_div(float2 a, float s) { return make_float2
 constexpr int WC_THREADS = 640;
 constexpr int WC_REGS = 40;
 
-__global__ void __maxnreg__(WC_REGS) wc_rk2_kernel(const float* __restrict__ m_in, const float* __restrict__ r_in,
-                                                   float* __restrict__ m_out, float* __restrict__ r_out,
+__global__ void __maxnreg__(WC_REGS) wc_rk2_kernel(const float* m_in, const float* r_in, float* m_out, float* r_out,
                                                    const WCParams P, const __grid_constant__ PdeBCRules Ru,
                                                    const __grid_constant__ PdeBCRules Rr) {
   extern __shared__ __align__(16) float sm[];
