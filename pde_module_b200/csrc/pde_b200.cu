@@ -707,6 +707,29 @@ int heat3d_split_run(const float* u_in, float* u_out, float* work, const Geo& G,
   return PDE_OK;
 }
 
+// Tile of the shared-memory 2D kernels for regions grown by H cells; false when its
+// region (two levels) does not fit.  Automatic shape: square tiles of about one per SM
+// (sides 16..64, balanced against the SM count); 16x32 tiles when those do not fit.
+bool heat2d_tile(const Geo& G, int ncomp, int H, int* tbx, int* tby) {
+  const size_t most = 227 * 1024 - sizeof(PdeBCRules);
+  auto bytes = [&]() { return (size_t)2 * (*tbx + 2 * H) * (*tby + 2 * H) * ncomp * sizeof(float); };
+  if (g_tile2d[0] > 0) {  // pde_set_launch_2d
+    *tbx = g_tile2d[0];
+    *tby = g_tile2d[1];
+  } else {
+    const int X = (int)G.n[0], Y = (int)G.n[1];
+    int t = (int)ceil(sqrt((double)X * Y / sm_count()));
+    t = t < 16 ? 16 : (t > 64 ? 64 : t);
+    *tbx = *tby = t;
+    balance_tiles(X, Y, tbx, tby);
+    if (bytes() > most) {
+      *tbx = 16;
+      *tby = 32;
+    }
+  }
+  return bytes() <= most;
+}
+
 // The fused rollout; time-dependent groups only when `allow_ramp`; step n of
 // the call fills the boundary at fp32(t0 + (n0 + n) * tstep).
 int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid* grid, int32_t ncomp,
@@ -730,13 +753,16 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
   const int R = W.radius;
   const bool two_d = (G.ndims == 2 && G.n[2] == 1);
   const bool s3d = !two_d && heat3d_ok(G, ncomp);
+  int k = heat_depth(G, ncomp, steps_per_pass);
+  if (k > nsteps) k = nsteps;
+  int tbx = 0, tby = 0;
+  // a depth is refused by one limit, whichever kernel would run
+  if (two_d && !heat2d_tile(G, ncomp, k * R + 1, &tbx, &tby)) return PDE_ERR_TOO_LARGE;
   if (two_d && g_dispatch != PDE_DISPATCH_GENERIC && rt_heat_shape(G, ncomp, rules)) {
     const RTPlan L = rt_heat_plan(G, nsteps, steps_per_pass, g_tile2d[0], g_tile2d[1]);
     if (L.ok)
       return rt_heat_run(L, u_in, u_out, work, G, W, *rules, alpha, dt, nsteps, t0, tstep, n0, st);
   }
-  int k = heat_depth(G, ncomp, steps_per_pass);
-  if (k > nsteps) k = nsteps;
   // a depth left open streams one step per pass on any shape (odd sides too, where the
   // quad-row map takes 43 us a step on 255 x 191 x 319 against 163 of the blocked kernel)
   if (s3d && (steps_per_pass == 0 || k == 1) && heat_stream_shape(G, ncomp) && aligned16(u_in) && aligned16(u_out) && aligned16(work))
@@ -761,23 +787,8 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
       H2Params P;
       P.X = (int)G.n[0]; P.Y = (int)G.n[1]; P.g = G.g; P.N = ncomp; P.k = ks;
       const int H = k * R + 1;  // must match heat2d_tb_kernel
-      // Automatic shape: square tiles of about one per SM (sides 16..64, balanced
-      // against the SM count), 512 threads; 16x32 tiles when those regions would
-      // not fit in shared memory.
-      int threads = g_threads2d > 0 ? g_threads2d : 512;
-      if (g_tile2d[0] > 0) {  // pde_set_launch_2d
-        P.TBX = g_tile2d[0];
-        P.TBY = g_tile2d[1];
-      } else {
-        int t = (int)ceil(sqrt((double)P.X * P.Y / sm_count()));
-        t = t < 16 ? 16 : (t > 64 ? 64 : t);
-        P.TBX = P.TBY = t;
-        balance_tiles(P.X, P.Y, &P.TBX, &P.TBY);
-        if ((size_t)2 * (P.TBX + 2 * H) * (P.TBY + 2 * H) * ncomp * sizeof(float) > 227 * 1024 - sizeof(PdeBCRules)) {
-          P.TBX = 16;
-          P.TBY = 32;
-        }
-      }
+      const int threads = g_threads2d > 0 ? g_threads2d : 512;
+      heat2d_tile(G, ncomp, H, &P.TBX, &P.TBY);
       P.RXM = P.TBX + 2 * H; P.RYM = P.TBY + 2 * H;
       P.tiles_y = (P.Y + P.TBY - 1) / P.TBY;
       const int tiles = ((P.X + P.TBX - 1) / P.TBX) * P.tiles_y;
@@ -785,7 +796,6 @@ int heat_rollout_run(const float* u_in, float* u_out, float* work, const PdeGrid
       P.alpha = alpha; P.dt = dt;
       P.t0 = t0; P.tstep = tstep; P.n0 = n0 + done;
       const size_t smem = (size_t)2 * P.RXM * P.RYM * ncomp * sizeof(float);
-      if (smem > 227 * 1024 - sizeof(PdeBCRules)) return PDE_ERR_TOO_LARGE;
       // one component and at most 8 region cells per thread: the register cell-list kernel
       const long long cap = (long long)P.RXM * P.RYM;
       const int cpt = (ncomp == 1 && cap < (1 << 16)) ? (cap <= 4LL * threads ? 4 : cap <= 8LL * threads ? 8 : 0) : 0;
@@ -1409,11 +1419,6 @@ int jacobi_setup(const Geo& G, float h2, int nsweeps, int k, bool only, int own_
                  const PdeBCRules& rules, JacobiLaunch* L) {
   L->run = JacobiRun{(int)G.n[0], (int)G.n[1], G.g, own_lo, own_hi, held_lo, held_hi, h2};
   L->rt.ok = false;
-  if (rt_fills_all_faces(rules)) L->rt = rt_jacobi_plan(L->run, nsweeps, k, only, g_tile2d[0], g_tile2d[1]);
-  if (L->rt.ok) {
-    L->k = L->rt.k;
-    return PDE_OK;
-  }
   L->k = k > 0 ? k : 10;
   if (L->k > nsweeps && nsweeps > 0) L->k = nsweeps;
   J2Params* JP = &L->JP;
@@ -1427,7 +1432,12 @@ int jacobi_setup(const Geo& G, float h2, int nsweeps, int k, bool only, int own_
   JP->h2 = h2;
   L->tiles = ((own_hi - own_lo + JP->TBX - 1) / JP->TBX) * JP->tiles_y;
   L->smem = (size_t)3 * JP->RXM * JP->RYM * sizeof(float);  // two levels and the rhs per cell
-  if (L->smem > 227 * 1024) return PDE_ERR_TOO_LARGE;
+  if (L->smem > 227 * 1024) return PDE_ERR_TOO_LARGE;  // the one limit of a depth, whichever kernel runs
+  if (rt_fills_all_faces(rules)) L->rt = rt_jacobi_plan(L->run, nsweeps, k, only, g_tile2d[0], g_tile2d[1]);
+  if (L->rt.ok) {
+    L->k = L->rt.k;
+    return PDE_OK;
+  }
   if (cudaFuncSetAttribute((const void*)jacobi2d_tb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) !=
       cudaSuccess)
     return PDE_ERR_CUDA;
