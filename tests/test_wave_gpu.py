@@ -146,3 +146,25 @@ def _pair_vs_separate(nf, na, k):
         assert torch.equal(lf[s][ins], lf_ref[s][ins]), s
     assert torch.equal(g, g_ref)
     assert torch.equal(q1, r1) and torch.equal(q2, r2)
+
+
+@pytest.mark.parametrize("shape", [(40, 44), (70, 131)])
+def test_zeros_keep_their_sign(shape):
+    """Cells at rest where K is 0: 2 u - u_prev + K L(u) is +0 + (-0) there where L(u) < 0,
+    and stays +0, in the forward and in the adjoint; compared as bits."""
+    rng = np.random.default_rng(shape[0])
+    X, Y = shape
+    dx, N = 1.0 / (X - 3), 11
+    K = (0.1 * dx * dx * (1.0 + rng.random((X, Y, 1, 1)))).astype(np.float32)
+    K[rng.random(K.shape) < 0.3] = 0.0
+    sparse = lambda: (rng.standard_normal(K.shape) * (rng.random(K.shape) < 0.3)).astype(np.float32) + np.float32(0.0)
+    u0, grad = sparse(), sparse()
+    solver = WaveSolver((X, Y, 1), dx, N)
+    Kd = torch.from_numpy(K).cuda()
+    uN = solver.forward(Kd, torch.from_numpy(u0).cuda())
+    _, gu = solver.backward(Kd, torch.from_numpy(grad).cuda())
+    st = fdm.wave_forward(K, u0, None, None, N, dx)
+    _, mu0, mu1 = fdm.wave_adjoint(K, st, grad, dx)
+    bits = lambda a: np.ascontiguousarray(a).view(np.int32)
+    assert np.array_equal(bits(uN.cpu().numpy()[:, :, 0, 0]), bits(st[-1]))
+    assert np.array_equal(bits(gu.cpu().numpy()[:, :, 0, 0]), bits(mu0 - mu1))
