@@ -5,10 +5,9 @@
 // which the state is 0), sized per grid so that its windows are filled.  A block of
 // 8 warps with 4 x 8 cells a thread (a 64 x 128 window) takes 128 registers a
 // thread: two blocks per SM, one loading or waiting while the other steps.  Bound by
-// issue (half the slots used, the fp32 pipe 43% busy in a capture).  On one B200,
-// against the shared-memory items, depth 10 the fastest of 4..16 for both: 64 heat
-// grids of 64..1024 a side x 100 steps 5.48 -> 2.04 ms, 24 wave grids x 200 steps
-// 3.02 -> 1.28 ms.
+// issue.  On one B200, against the shared-memory items, depth 10 the fastest of 4..16
+// for both: 64 heat grids of 64..1024 a side x 100 steps 5.48 -> 2.04 ms, 24 wave
+// grids x 200 steps 3.02 -> 1.28 ms.
 #pragma once
 #include "batched.cuh"
 #include "regtile.cuh"
@@ -212,16 +211,24 @@ __global__ void __launch_bounds__(BRT_WARPS * 32, 2) batched_rt_kernel(const Bat
         rt_store<C, RPT>(u, (swapped ? out1 : out0) + first, Gd.Y, V);
         rt_store<C, RPT>(um, (swapped ? out0 : out1) + first, Gd.Y, V);
       }
-      // The last block writes the caller's fields: 0 on the ring and the ghosts, which
-      // no window holds, so the tiles at the box's edges may write them at any time.
-      if (tb == P.ntb - 1 && (V.bx0 == 0 || V.by0 == 0 || V.bx1 == W.BX || V.by1 == W.BY)) {
+      // The caller's fields come back 0 on the ring and the ghosts.  No window holds
+      // those cells, so the tiles at the box's edges may write them at any time: in
+      // the first block, away from the launch's tail (24 grids x 200 steps: 1.302 ms
+      // by a walk over the grown tile in the last block, 1.280 ms so).
+      if (tb == 0) {
         const int x0 = V.bx0 + pad, x1 = V.bx1 + pad, y0 = V.by0 + pad, y1 = V.by1 + pad;  // the tile in the array
-        const int ax = V.bx0 == 0 ? 0 : x0, bx = V.bx1 == W.BX ? Gd.X : x1;
-        const int ay = V.by0 == 0 ? 0 : y0, by = V.by1 == W.BY ? Gd.Y : y1;
-        RectWalk wk(by - ay, (int)blockDim.x);
-        for (int i = tid; i < (bx - ax) * (by - ay); i += (int)blockDim.x, wk.next()) {
-          const int x = ax + wk.row, y = ay + wk.col;
-          if (x < x0 || x >= x1 || y < y0 || y >= y1) out0[(size_t)x * Gd.Y + y] = out1[(size_t)x * Gd.Y + y] = 0.0f;
+        const int top = V.bx0 == 0 ? x0 : 0, bottom = V.bx1 == W.BX ? Gd.X - x1 : 0;
+        const int left = V.by0 == 0 ? y0 : 0, right = V.by1 == W.BY ? Gd.Y - y1 : 0;
+        const int wide = left + (y1 - y0) + right, rows_out = top + bottom, cols_out = left + right;
+        for (int i = tid; i < rows_out * wide; i += (int)blockDim.x) {  // the rows above and below, corners included
+          const int r = i / wide, x = r < top ? r : x1 + r - top;
+          const size_t c = (size_t)x * Gd.Y + y0 - left + (i - r * wide);
+          Gd.a0[c] = Gd.a1[c] = 0.0f;
+        }
+        for (int i = tid; i < (x1 - x0) * cols_out; i += (int)blockDim.x) {
+          const int r = i / cols_out, q = i - r * cols_out, y = q < left ? q : y1 + q - left;
+          const size_t c = (size_t)(x0 + r) * Gd.Y + y;
+          Gd.a0[c] = Gd.a1[c] = 0.0f;
         }
       }
     }
