@@ -1287,17 +1287,18 @@ def run_profile_heat3d(args):
 def run_profile_2d(args):
     """The 2D time-stepping kernels for profilers, eager (no graphs), short runs:
     wave    - 512^2 wave problem, 96 steps, forward + adjoint (k = 8, automatic tile)
-    heat    - 256^2 fused heat rollout (Dirichlet 0), 96 steps (k = 8, automatic launch shape)
-    heatadj - 256^2 heat, alpha field, 96 steps, forward + adjoint (k = 4)
-    batched - the 64-grid batched heat rollout, 16 steps (k = 4, 64 x 64 tiles)
-    ldc     - the 1024^2 lid-driven cavity, 4 steps (50 Jacobi sweeps each)"""
+    heat    - 256^2 fused heat rollout (Dirichlet 0), 96 steps
+    heatadj - 256^2 heat, alpha field, 96 steps, forward + adjoint
+    batched - the 64-grid batched heat rollout, 20 steps
+    ldc     - the 1024^2 lid-driven cavity, 4 steps (50 Jacobi sweeps each)
+    All at the depths and launch shapes the library chooses."""
     import torch
     import pde_module_b200 as P
     from pde_module_b200.time_step import wave as W
     t0 = time.time()
     for _ in range(args.iters):
         if args.profile_op == "wave":
-            solver, c, u0, target, dt, mask = W.make_problem(n=512, nsteps=96, steps_per_pass=8)
+            solver, c, u0, target, dt, mask = W.make_problem(n=512, nsteps=96)
             solver.graphs = False
             solver.set_checkpoint_every(None)
             K = (dt * dt) * c * c
@@ -1309,14 +1310,14 @@ def run_profile_2d(args):
             u0 = torch.rand((n + 2, n + 2, 1, 1), device="cuda")
             bc = P.GridBoundary(u0, dx, g)
             bc.dirichlet_BC("ALL", 0.0)
-            P.HeatRollout(bc, dx, 1.0, 0.2 * dx * dx, steps_per_pass=8)(u0, 96)
+            P.HeatRollout(bc, dx, 1.0, 0.2 * dx * dx)(u0, 96)
         elif args.profile_op == "heatadj":
             n, g = 256, 1
             dx = 1.0 / n
             u0 = torch.rand((n + 2, n + 2, 1, 1), device="cuda")
             bc = P.GridBoundary(u0, dx, g)
             bc.dirichlet_BC("ALL", 0.0)
-            solver = P.HeatSolver(bc, dx, 0.2 * dx * dx, 96, steps_per_pass=4, graphs=False)
+            solver = P.HeatSolver(bc, dx, 0.2 * dx * dx, 96, graphs=False)
             a = torch.ones_like(u0)
             uN = solver.forward(a, u0)
             solver.backward(a, uN)
@@ -1326,8 +1327,8 @@ def run_profile_2d(args):
         else:
             sides, alpha, u0, dx, dt = batched_problem()
             fields = [torch.from_numpy(u[:, :, None, None]).cuda() for u in u0]
-            roll = P.BatchedHeatRollout(fields, dx, alpha, dt, tile=(64, 64), steps_per_pass=4)
-            roll(16)
+            roll = P.BatchedHeatRollout(fields, dx, alpha, dt)
+            roll(20)
     torch.cuda.synchronize()
     print(json.dumps({"profile_op": args.profile_op, "iters": args.iters, "s": round(time.time() - t0, 3)}))
     return 0

@@ -231,10 +231,12 @@ int pde_bc_compile(const PdeBCGroup* groups, int32_t ngroups, const PdeGrid* gri
  * boundary-filled values of the last step (the unfused chain leaves the same values
  * when the Laplacian output's ghost cells are zero).
  * u_in: initial field; u_out: result; work: scratch of the same size (used as the
- * ping-pong buffer when nsteps > steps_per_pass).  u_out may equal u_in.
+ * ping-pong buffer when one pass does not do).  u_out may equal u_in.
  * steps_per_pass: temporal-blocking depth k (0 = choose).  2D (Z == 1) scalar
- * grids with every face filled hold their windows in registers, k steps per pass
- * (chosen by a cost model); other 2D grids use shared-memory tiles (0 = 8).  3D
+ * grids with every face filled hold their windows in registers; there k is the
+ * deepest pass allowed, and a cost model takes the depth that is fastest under it
+ * (0: under 25).  Other 2D grids use shared-memory tiles at exactly k (0 = 8).  A
+ * depth whose shared-memory region does not fit is PDE_ERR_TOO_LARGE on both.  3D
  * scalar fields with at least 3 interior cells per axis and 16-byte aligned buffers
  * run, at 0 or 1, a surface fill and the TMA streaming heat step per step; deeper
  * requests, and fields of several components, stream along X with k steps per pass
@@ -311,7 +313,11 @@ typedef struct PdeLDCParams {
   float   nu;               /* kinematic viscosity                              */
   float   dt;               /* time step                                        */
   int32_t jacobi_iters;     /* pressure sweeps per step                         */
-  int32_t jacobi_per_pass;  /* sweeps per launch (temporal blocking), 0 = 10    */
+  int32_t jacobi_per_pass;  /* sweeps per launch (temporal blocking): the most of a pass
+                               of pde_ldc_rollout, 0 = chosen by a cost model (10 where
+                               the sweeps run from shared memory); too deep a pass for
+                               shared memory is PDE_ERR_TOO_LARGE.  Slabs run exactly
+                               the sweeps each call asks for */
 } PdeLDCParams;
 
 /* nsteps of the projection method on a 2D grid, u (X,Y,1,2) and p (X,Y,1,1)
@@ -428,19 +434,20 @@ int pde_wave_pair(const float* K, const float* u_prev, const float* u_cur, int32
 /* Launch shape of the tiled 2D kernels of pde_heat_rollout[_at],
  * pde_heat_forward, pde_heat_adjoint, pde_wave_forward, pde_wave_adjoint,
  * pde_wave_pair, pde_wc_rk2 and the Jacobi sweeps of pde_ldc_rollout and
- * pde_ldc_slab_step, process-wide:
- * output tile (sides 8..256; (0, 0) = automatic: the largest of 32x64, 32x32,
- * 16x32 that gives every SM a tile, enlarged slightly when the count is just
- * above a multiple of the SM count; for the fused heat rollout square tiles of
- * about one per SM, sides 16..64) and threads per block (256, 512, 1024;
- * 0 = automatic: for the wave and differentiable-heat kernels 1024 with up to one
- * tile per SM, 512 up to two, else 256; 512 for the fused heat rollout and the
- * weakly compressible step (which takes 256 or 512); 256 for the Jacobi sweeps).
- * The Jacobi sweeps with both left automatic take one near-square tile per SM
- * and 1024 threads when those tiles have sides of at least 32 and their region
- * holds at most 12 cells per thread.  Any shape whose region holds at most 12
- * cells per thread runs the register cell-list Jacobi kernel, others the
- * flat-walk kernel (same results). */
+ * pde_ldc_slab_step, process-wide; results do not depend on it.
+ * Output tile (sides 8..256; (0, 0) = automatic).  Calls that run on register tiles
+ * take a given tile where a window holds it with its halo, and the shared-memory
+ * kernels otherwise; left automatic, the cost model chooses window and tile.  The
+ * shared-memory kernels' automatic tile: the largest of 32x64, 32x32, 16x32 that
+ * gives every SM a tile, enlarged slightly when the count is just above a multiple of
+ * the SM count; for the fused heat rollout square tiles of about one per SM, sides
+ * 16..64; for the weakly compressible step squares of 8 to 32, the smallest that are
+ * resident together.
+ * Threads per block (256, 512, 1024; 0 = automatic) of the shared-memory kernels;
+ * register tiles follow their window and ignore it.  Automatic: 1024 for the wave and
+ * differentiable-heat kernels with up to one tile per SM, 512 up to two, else 256; 512
+ * for the fused heat rollout; 256 for the Jacobi sweeps; for the weakly compressible
+ * step a thread per cell of the region up to 640, else 512 (it takes 256 or 512). */
 int pde_set_launch_2d(int32_t tile_x, int32_t tile_y, int32_t threads);
 
 /* Launch shape of the 3D streaming heat rollout (pde_heat_rollout[_at] on 3D

@@ -4,8 +4,8 @@
 // cover each grid's stencil box (wave: the cells inside the node ring, outside of
 // which the state is 0), sized per grid so that its windows are filled.  A block of
 // 8 warps with 4 x 8 cells a thread (a 64 x 128 window) takes 128 registers a
-// thread: two blocks per SM, one loading or waiting while the other steps.  Bound by
-// issue.  On one B200, against the shared-memory items, depth 10 the fastest of 4..16
+// thread: two blocks per SM, one loading or waiting while the other steps.  Half the
+// issue slots are used (barriers, dependent sums, window loads).  On one B200, against the shared-memory items, depth 10 the fastest of 4..16
 // for both: 64 heat grids of 64..1024 a side x 100 steps 5.48 -> 2.04 ms, 24 wave
 // grids x 200 steps 3.02 -> 1.28 ms.
 #pragma once

@@ -65,7 +65,6 @@ struct RTView {
     llo = ylo && lane == 0;
     lhi = yhi && lane == lh;
   }
-  __device__ bool in_tile(int x, int y) const { return x >= bx0 && x < bx1 && y >= by0 && y < by1; }
   __device__ bool row_in(int r) const { return r0 + r >= bx0 && r0 + r < bx1; }           // the same for the whole warp
   __device__ bool col_in(int j) const { return on && c0 + j >= by0 && c0 + j < by1; }
 };
@@ -694,8 +693,8 @@ struct RJParams {
 };
 
 // k sweeps  p <- 0.25 * ((((pW + pE) + pS) + pN) - h^2 rhs)  of a pass on BC_p(p);
-// h^2 rhs stays in registers.  Bound by issue (arithmetic, shuffles and row exchange
-// share the slots).  50 sweeps on one B200, against cell lists over shared memory
+// h^2 rhs stays in registers.  Bound by a sweep's latency (barrier, dependent sums) with
+// 41% of the issue slots used.  50 sweeps on one B200, against cell lists over shared memory
 // (five words of it read and one written per cell and sweep): 1024^2 139 -> 60 us
 // (one 128 x 128 window per SM, 4 x 8 cells a thread), 400^2 31 us, 100^2 24 us.
 template <int C, int RPT>

@@ -2,10 +2,10 @@
 // adjoint, and both in one launch (wave.cuh states the scheme and the order of
 // operations).  Against the interleaved shared-memory regions (three to seven words a
 // cell, read five times a step), 512^2 x 2000 steps on one B200: forward 2.3 -> 1.3
-// ms, recomputation and adjoint 4.2 -> 3.6 ms.  Bound by issue and by what a pass
-// spends besides its steps (launch, loading and storing seven fields' windows); the
-// forward takes up to 16 steps a pass, both together 8.  Tiles cover the cells inside the node ring, outside of which every
-// state is 0.
+// ms, recomputation and adjoint 4.2 -> 3.6 ms.  Bound by the latency of a step (37-43% of
+// the issue slots used) and by what a pass spends besides its steps (launch, loading and
+// storing seven fields' windows); the forward takes up to 16 steps a pass, both together
+// 8.  Tiles cover the cells inside the node ring, outside of which every state is 0.
 #pragma once
 #include "regtile.cuh"
 

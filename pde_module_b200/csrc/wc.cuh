@@ -93,8 +93,9 @@ __device__ __forceinline__ float2 wc_div(float2 a, float s) { return make_float2
 // one, so an interior tile meets five barriers a step and an edge tile eleven (14 and
 // 22 when every operator was its own phase).  Both components of a vector move in one
 // 8-byte access: a cell's f takes 19 shared-memory loads instead of 34 with two-way
-// bank conflicts.  Latency bounds a step on small grids (201^2 nodes: 15.7 -> 8.9 us a
-// step), the loads and the arithmetic on large ones (1025^2: 73.7 -> 62.0 us).  An array
+// bank conflicts.  Latency bounds a step on small grids (201^2 nodes, calls of 100 steps:
+// 10.2 -> 6.5 us a step), the loads and the arithmetic on large ones (1025^2: 73.7 ->
+// 61.7 us).  An array
 // of its own for y1's velocity saves one more barrier but 1.5% only, and costs a block
 // per SM.
 // WC_REGS: 3 blocks of 512 threads per SM.
