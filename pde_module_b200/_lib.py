@@ -246,6 +246,8 @@ def make_grid(shape3, ghost_cells: int, order: int, dx: float) -> PdeGrid:
 def stream_ptr(t: torch.Tensor | None = None) -> int:
     # The raw handle: a torch.cuda.Stream object around it costs 2 us of each call.
     dev = t.get_device() if t is not None else torch.cuda.current_device()
+    if dev < 0:
+        raise ValueError(f"expected a tensor on a cuda device, but got: {t.device}")
     return torch._C._cuda_getCurrentRawStream(dev)
 
 

@@ -255,3 +255,17 @@ def test_wave_pair_validation_needs_no_gpu():
     assert call(cell=5) == _lib.PDE_ERR_ARG          # a source cell needs source samples
     assert call(nf=0, na=0) == _lib.PDE_OK           # nothing to do
     assert call(nf=0, lf=None, up=None, uc=None, na=0) == _lib.PDE_OK
+
+
+def test_a_cpu_tensor_has_no_stream(monkeypatch):
+    """Entry points without a check of their own (the cavity, the slabs) are kept from
+    passing host memory to a kernel by this."""
+    import torch
+    asked = []
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda i: asked.append(i) or 0, raising=False)
+    with pytest.raises(ValueError, match="cuda"):
+        _lib.stream_ptr(torch.zeros(1))
+    from pde_module_b200 import FractionalStepLDC
+    with pytest.raises(ValueError, match="cuda"):
+        FractionalStepLDC(n=8, device="cpu").step()
+    assert not asked
